@@ -207,7 +207,8 @@ def prepare(case: dict, seed: int) -> dict:
         state["out"] = (np.empty(shape, np.float32) if case["host"]
                         else torch.empty(shape, dtype=torch.float32, device="cuda"))
     elif kind == "batch":
-        g = np.random.default_rng(seed)
+        # the jobs' sizes are the case's, their scenes the seed's
+        g = np.random.default_rng(case["size"])
         sids, sts, outs = [], [], []
         for k in range(case["size"]):
             n = int(np.exp(g.uniform(np.log(10), np.log(50_000))))
