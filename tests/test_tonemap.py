@@ -68,3 +68,27 @@ def test_device_tonemap_rejects_bad_arguments(gpu):
         gpu.tonemap(np.zeros((2, 2, 3), np.float32), tonemap=3)
     assert e.value.code == A.ERR_UNSUPPORTED
     assert gpu.tonemap(np.zeros((0, 3), np.float32)).shape == (0, 3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("pixels", [1, 5, 6, 16, 341, 4097])
+@pytest.mark.parametrize("skip_in,skip_out", [(0, 0), (1, 1), (3, 7), (2, 18), (1, 0)])
+def test_device_buffers_of_any_size_and_alignment(gpu, pixels, skip_in, skip_out):
+    """Ragged channel counts, and buffers whose 16-byte boundaries lie
+    together at the front, later, or never (1, 0): the host's bytes, and
+    nothing written beside them."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(pixels)
+    hdr = np.exp(rng.normal(-1, 1.5, (pixels, 3))).astype(np.float32)
+    hdr[0] = (np.nan, 2.0 ** -20, np.nextafter(np.float32(2.0 ** -20), np.float32(0)))
+    d_in = torch.zeros(3 * pixels + 8, dtype=torch.float32, device="cuda")
+    d_in[skip_in:skip_in + 3 * pixels] = torch.from_numpy(hdr.reshape(-1)).cuda()
+    d_out = torch.full((3 * pixels + 64,), 77, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    gpu.check(gpu.lib.pgpu_tonemap(gpu.h, d_in.data_ptr() + 4 * skip_in, pixels, A.TONEMAP_NONE,
+                                   0.0, A.TONEMAP_DEVICE_INPUT | A.TONEMAP_DEVICE_OUTPUT,
+                                   d_out.data_ptr() + skip_out), "pgpu_tonemap")
+    got = d_out.cpu().numpy()
+    want = O.rgb8(np.nan_to_num(hdr, nan=0.0), tonemap=A.TONEMAP_NONE).reshape(-1)
+    assert np.array_equal(got[skip_out:skip_out + 3 * pixels], want)
+    assert (got[:skip_out] == 77).all() and (got[skip_out + 3 * pixels:] == 77).all()
