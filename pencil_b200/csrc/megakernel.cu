@@ -24,9 +24,27 @@ constexpr int kMkShared = 16;   // stack entries per thread kept in shared memor
 // 382.3 ms.
 constexpr int kMkMinBlocks = 8;
 
-template <bool COUNT, bool TREE, bool PIXEL_SEQ, bool WIDE>
+// Pixels per warp of the reference-exact mode (Pencil's per-pixel stream, both
+// glass branches). A launch too small to fill the GPU (a worker's 64x64 tile
+// has 4096 pixels) ends with its longest path, a serial chain of node loads
+// through glass. Such a launch gives each pixel a team of lanes that trace
+// the shadow rays of its vertices side by side, as long as its warps fit the
+// GPU at once (32 on each of 148 SMs, what 64 registers allow). Teams of 8: a
+// 64x64 tile of six rooms of 63 primitives took 4.12 / 0.67 / 1.13 / 12.2 /
+// 1.36 / 6.5 ms with one lane per pixel, 1.93 / 0.45 / 0.67 / 5.4 / 0.73 / 3.3
+// with 8 (6 shadow rays a vertex), 2.82 / 0.90 / 0.98 / 6.1 / 1.02 / 2.9 with
+// 32: more warps than a team can use only take issue slots from each other.
+constexpr long long kTeamWarps = 148 * 32;
+constexpr int kMaxTeam = 8;
+static int pixels_per_warp(long long pixels) {
+    int per = 32 / kMaxTeam;
+    while (per < 32 && (pixels + per - 1) / per > kTeamWarps) per *= 2;
+    return per;
+}
+
+template <bool COUNT, bool TREE, bool PIXEL_SEQ, bool WIDE, bool COOP>
 __global__ void __launch_bounds__(128, kMkMinBlocks)
-mk_render(SceneView S, PathParams P, int G, float* __restrict__ out, float* __restrict__ m2,
+mk_render(SceneView S, PathParams P, int G, int per_warp, float* __restrict__ out, float* __restrict__ m2,
           unsigned long long* __restrict__ counters) {
     extern __shared__ int smem[];
     TravStack<kMkShared> stk;
@@ -34,9 +52,10 @@ mk_render(SceneView S, PathParams P, int G, float* __restrict__ out, float* __re
     stk.st = reinterpret_cast<float*>(smem + kMkShared * blockDim.x) + threadIdx.x;
     stk.stride = blockDim.x;
     RayCount rc = {};
-    Tracer<kMkShared, COUNT, WIDE> tr{S, P, stk, rc};
-
-    const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    // COOP: a team of 32 / per_warp lanes for each of the warp's pixels
+    const int team = COOP ? 32 / per_warp : 1;
+    Tracer<kMkShared, COUNT, WIDE, COOP> tr{S, P, stk, rc, team};
+    const long long gid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / team;
     const bool tile = P.tile_w > 0;
     const int outW = tile ? P.tile_w : P.W, outH = tile ? P.tile_h : P.H;
     const long long npix = (long long)outW * outH;
@@ -78,7 +97,7 @@ mk_render(SceneView S, PathParams P, int G, float* __restrict__ out, float* __re
         acc2.y += __shfl_xor_sync(0xffffffffu, acc2.y, off);
         acc2.z += __shfl_xor_sync(0xffffffffu, acc2.z, off);
     }
-    if (active && lane_g == 0) {
+    if (active && lane_g == 0 && (!COOP || threadIdx.x % team == 0)) {
         const float denom = (float)P.spp;
         out[3 * pix + 0] = acc.x / denom;
         out[3 * pix + 1] = acc.y / denom;
@@ -106,10 +125,19 @@ static cudaError_t launch_mk(const SceneView& S, const PathParams& P, int G, flo
                              float* m2, unsigned long long* counters, cudaStream_t st) {
     const int block = 128;
     long long threads = (P.tile_w > 0 ? (long long)P.tile_w * P.tile_h : (long long)P.W * P.H) * G;
-    long long blocks = (threads + block - 1) / block;
-    size_t smem = (size_t)kMkShared * block * 8;
-    mk_render<COUNT, TREE, PIXEL_SEQ, WIDE><<<(unsigned)blocks, block, smem, st>>>(S, P, G, out,
-                                                                                     m2, counters);
+    const size_t smem = (size_t)kMkShared * block * 8;
+    auto grid = [&](long long n) { return (unsigned)((n + block - 1) / block); };
+    if constexpr (TREE && PIXEL_SEQ && !COUNT) {
+        const int per_warp = pixels_per_warp(threads);
+        if (per_warp < 32) {
+            mk_render<COUNT, TREE, PIXEL_SEQ, WIDE, true>
+                <<<grid(threads * (32 / per_warp)), block, smem, st>>>(S, P, G, per_warp, out, m2,
+                                                                       counters);
+            return cudaGetLastError();
+        }
+    }
+    mk_render<COUNT, TREE, PIXEL_SEQ, WIDE, false><<<grid(threads), block, smem, st>>>(
+        S, P, G, 32, out, m2, counters);
     return cudaGetLastError();
 }
 

@@ -333,12 +333,57 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& S, const PathParam
 // the 4-wide tree the wavefront walks (ClosestTrav4/AnyTrav4); otherwise
 // Pencil's binary tree (the tree BVHNode::hit walks, src/bvh.hpp:31-48) in
 // its child-pair layout, nearest child first.
-template <int kShared, bool COUNT, bool WIDE = false>
+// COOP: the path belongs to a group of `team` lanes of one warp (a power of
+// two, aligned) that hold the same state and take every step together; the
+// shadow rays of a vertex are shared out among them, one each, and their
+// terms summed in the order one lane would have summed them.
+template <int kShared, bool COUNT, bool WIDE = false, bool COOP = false>
 struct Tracer {
     const SceneView& S;
     const PathParams& P;
     TravStack<kShared>& stk;
     RayCount& rc;
+    int team = 1;
+
+    // Shadow samples of a vertex waiting to be traced by the group: lane q of
+    // the group holds sample q.
+    struct Team {
+        V3 L;
+        float tmax, w;
+        int light, group_end;
+        int n = 0;
+    };
+    __device__ __forceinline__ int team_lane() const { return (threadIdx.x & 31) & (team - 1); }
+    __device__ __forceinline__ void put(Team& t, V3 L, float tmax, float w, int light, int ge) {
+        if (t.n == team_lane()) {
+            t.L = L;
+            t.tmax = tmax;
+            t.w = w;
+            t.light = light;
+            t.group_end = ge;
+        }
+        ++t.n;
+    }
+    // Traces the waiting samples, one per lane; add(c, group_end, visible) is
+    // then called for each in order with term()'s value on its lane.
+    template <class Term, class Add>
+    __device__ __forceinline__ void drain(Team& t, V3 sorg, Term term, Add add) {
+        const int me = team_lane(), base = (threadIdx.x & 31) & ~(team - 1);
+        const unsigned mask = (team == 32 ? 0xffffffffu : ((1u << team) - 1u)) << base;
+        bool vis = false;
+        V3 c = v3(0, 0, 0);
+        if (me < t.n) {
+            vis = S.lights[t.light].is_emissive || !occluded(Ray{sorg, t.L}, P.bias, t.tmax);
+            if (vis) c = term(t);
+        }
+        const unsigned v = __ballot_sync(mask, vis) >> base;
+        for (int q = 0; q < t.n; ++q) {
+            const V3 cq = v3(__shfl_sync(mask, c.x, base + q), __shfl_sync(mask, c.y, base + q),
+                             __shfl_sync(mask, c.z, base + q));
+            add(cq, __shfl_sync(mask, t.group_end, base + q), ((v >> q) & 1u) != 0);
+        }
+        t.n = 0;
+    }
 
     __device__ __forceinline__ int closest(const Ray& r, Hit& h) {
         if (COUNT) rc.ext++;
@@ -363,6 +408,9 @@ struct Tracer {
                                 bool shade) {
         V3 albedo = ld3(m.albedo);
         V3 local = ld3(m.emission);
+        if constexpr (COOP) {
+            if (shade) return whitted_local_team(r, h, m, rng);
+        }
         for (int li = 0; li < S.n_lights; ++li) {
             const DevLight& l = S.lights[li];
             if (l.kind == 2) continue;
@@ -388,6 +436,49 @@ struct Tracer {
             }
             local = local + contrib / (float)ns;
         }
+        return local + albedo * ld3(S.amb);
+    }
+
+    // whitted_local by the lanes of a group: the same samples, each lane
+    // tracing and weighing its own.
+    __device__ V3 whitted_local_team(const Ray& r, const Hit& h, const DevMaterial& m, Rng& rng) {
+        const V3 albedo = ld3(m.albedo);
+        const V3 sorg = h.p + h.n * P.bias;
+        V3 local = ld3(m.emission), contrib = v3(0, 0, 0);
+        auto term = [&](const Team& t) {
+            const DevLight& l = S.lights[t.light];
+            float ndotl = clampf(dot(h.n, t.L), 0.0f, 1.0f);
+            V3 c = albedo * ld3(l.intensity) * ndotl;
+            if (m.specular > 0.0f && ndotl > 0.0f) {
+                V3 V = -normalized(r.d);
+                V3 H = normalized(t.L + V);
+                float ndoth = clampf(dot(h.n, H), 0.0f, 1.0f);
+                float spec = powf(ndoth, m.shininess);
+                c = c + ld3(m.specular_color) * ld3(l.intensity) * (spec * m.specular);
+            }
+            return c;
+        };
+        auto add = [&](V3 c, int group_end, bool visible) {
+            if (visible) contrib = contrib + c;
+            if (group_end > 0) {
+                local = local + contrib / (float)group_end;
+                contrib = v3(0, 0, 0);
+            }
+        };
+        Team t;
+        for (int li = 0; li < S.n_lights; ++li) {
+            const DevLight& l = S.lights[li];
+            if (l.kind == 2) continue;
+            const int ns = (l.radius > 0.0f) ? P.soft : 1;
+            for (int k = 0; k < ns; ++k) {
+                V3 L;
+                float dist;
+                light_dir(l, h.p, rng, L, dist);
+                put(t, L, dist - P.bias, 0.0f, li, k == ns - 1 ? ns : 0);
+                if (t.n == team) drain(t, sorg, term, add);
+            }
+        }
+        if (t.n) drain(t, sorg, term, add);
         return local + albedo * ld3(S.amb);
     }
 
@@ -534,6 +625,38 @@ struct Tracer {
     __device__ __forceinline__ void pt_direct(const Hit& h, const DevMaterial& m, V3 T, Rng& rng,
                                               V3& rad, bool quad_nee) {
         V3 albedo = ld3(m.albedo);
+        if constexpr (COOP) {
+            const V3 sorg = h.p + h.n * P.bias;
+            auto term = [&](const Team& t) {
+                const DevLight& l = S.lights[t.light];
+                if (l.kind == 2) return T * albedo * ld3(l.intensity) * t.w;
+                const float ndotl = clampf(dot(h.n, t.L), 0.0f, 1.0f);
+                return light_term(l, P.mis != 0, T, albedo, t.L, t.w, ndotl);
+            };
+            auto add = [&](V3 c, int, bool visible) {
+                if (visible) rad = rad + c;
+            };
+            Team t;
+            for (int quad = 0; quad < (quad_nee ? 2 : 1); ++quad) {
+                for (int li = 0; li < S.n_lights; ++li) {
+                    const DevLight& l = S.lights[li];
+                    if ((l.kind == 2) != (quad == 1)) continue;
+                    V3 L;
+                    float tmax, w;
+                    if (quad) {
+                        if (!quad_sample(l, h.p, h.n, sorg, P.bias, rng, L, tmax, w)) continue;
+                    } else {
+                        light_dir(l, h.p, rng, L, w);      // w: the distance
+                        tmax = w - P.bias;
+                    }
+                    put(t, L, tmax, w, li, 0);
+                    if (t.n == team) drain(t, sorg, term, add);
+                }
+            }
+            if (t.n) drain(t, sorg, term, add);
+            rad = rad + T * albedo * ld3(S.amb);
+            return;
+        }
         for (int li = 0; li < S.n_lights; ++li) {
             const DevLight& l = S.lights[li];
             if (l.kind == 2) continue;
