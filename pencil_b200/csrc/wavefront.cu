@@ -5,8 +5,10 @@
 // processed in chunks of whole pixels that fit the queue capacity Q. For each
 // chunk the kernels run
 //
-//   generate                          camera rays of every path in the chunk
-//   depth x { extend, shade, shadow } closest hit / shade_vertex / any hit
+//   camera                            camera rays of every path in the chunk
+//                                     and their closest hits
+//   depth x { extend, shade, shadow } closest hit (after the first bounce) /
+//                                     shade_vertex / any hit
 //   accumulate                        per-pixel sums in the megakernel's order
 //
 // extend, shade and shadow are persistent: a grid sized to fill the GPU whose
@@ -94,7 +96,14 @@ struct WfArgs {
     int* status;              // 1: shadow record overflow
     unsigned long long* counters;
     int sort_key;
-    int packets;              // 1: the first bounce of a one-scene frame as warp packets
+    int packets;              // 1: camera rays as warp packets (wf_camera)
+    // sort keys 0/1: the shadow kernel walks the list of slots with shadow work
+    // instead of the queue. A vertex with several records keeps its lane for
+    // several rays, and lanes that drift apart lose more by the list's order
+    // (Whitted room, six records, 1.2M paths: 1.16 ms of shadow rays on the
+    // queue, 1.39 on the list) than empty entries cost; with one or two
+    // records the entries cost more (batch of 32 clouds: 8.5 and 6.4 ms).
+    int shadow_list;
     int refill_below;         // extend/shadow: a warp refetches rays once at most
                               // this many of its lanes are still traversing
     // sort keys 2/3 (counting sort by sort_key_of of each iteration's shadow
@@ -240,6 +249,29 @@ __device__ __forceinline__ int fetch32(unsigned int* cursor) {
 }
 
 // ---- generate -----------------------------------------------------------------
+// The camera ray of a path and its generator after the jitter.
+struct CameraPath {
+    Ray ray;
+    Rng rng;
+};
+__device__ __forceinline__ CameraPath camera_path(const WfJob& J, const SceneView& S,
+                                                  long long path) {
+    const PathParams& P = J.P;
+    const long long local = path - J.path_off;
+    const int pix = (int)(local / P.spp);
+    const int s = (int)(local % P.spp);
+    // pixel of the image (of the job's window when it has one)
+    const int ww = P.tile_w > 0 ? P.tile_w : P.W;
+    const int i = pix % ww + P.tile_x, j = pix / ww + P.tile_y;
+    CameraPath c;
+    c.rng = Rng{path_seed(i, j, s + P.sample_offset, P.salt)};
+    float u, v;
+    sample_uv(i, j, s % P.n, s / P.n, P.W, P.H, P.n, c.rng, u, v);
+    c.ray = camera_ray(S.cam, u, v);
+    return c;
+}
+
+// Camera rays one per lane, for the frames that trace them so.
 template <bool COUNT, bool ONE>
 __global__ void __launch_bounds__(kWfMaxBlock)
 wf_generate(WfArgs A, long long path_begin, int n_slots) {
@@ -252,17 +284,9 @@ wf_generate(WfArgs A, long long path_begin, int n_slots) {
         const int jb = ONE ? 0 : find_job(A.jobs, A.n_jobs, path);
         const WfJob& J = job_of<ONE>(A, jb);
         const PathParams& P = J.P;
-        const SceneView& S = view_of<ONE>(A, jb);
-        long long local = path - J.path_off;
-        int pix = (int)(local / P.spp);
-        int s = (int)(local % P.spp);
-        // pixel of the image (of the job's window when it has one)
-        const int ww = P.tile_w > 0 ? P.tile_w : P.W;
-        int i = pix % ww + P.tile_x, j = pix / ww + P.tile_y;
-        Rng rng{path_seed(i, j, s + P.sample_offset, P.salt)};
-        float u, v;
-        sample_uv(i, j, s % P.n, s / P.n, P.W, P.H, P.n, rng, u, v);
-        Ray r = camera_ray(S.cam, u, v);
+        const CameraPath c = camera_path(J, view_of<ONE>(A, jb), path);
+        const Ray r = c.ray;
+        const Rng rng = c.rng;
         A.ray_o[slot] = make_float4(r.o.x, r.o.y, r.o.z, 0.0f);
         A.ray_d[slot] = make_float4(r.d.x, r.d.y, r.d.z, 0.0f);
         // a path's first shade (iteration 0) starts from T = 1, L = 0 without
@@ -374,11 +398,9 @@ __device__ __forceinline__ void warp_append(bool take, int slot, int* counter, i
 }
 
 // ---- extend, camera rays: warp packets --------------------------------------------
-// The first bounce's queue holds the camera rays in slot order, so a warp's
-// 32 rays are the samples of neighbouring pixels of one scene: nearly the same
-// ray (a batch's first queue is appended a generate warp at a time, so its
-// warps are mostly such groups too; a warp whose rays belong to different
-// scenes traces them one by one).
+// A warp makes the camera rays of 32 consecutive paths, the samples of
+// neighbouring pixels of one scene: nearly the same ray (in a batch a warp
+// whose paths belong to different scenes traces them one by one).
 // The warp traverses the wide tree once for all of them: every lane tests
 // every node the packet enters against its own ray and its own t_best, the
 // packet enters a child that any lane still reaches (nearest first by the
@@ -386,52 +408,61 @@ __device__ __forceinline__ void warp_append(bool take, int slot, int* counter, i
 // Node loads are broadcasts and all lanes stay busy. A lane still tests a
 // leaf only when its own slab test reaches it, so its result is the closest
 // hit among the same leaves as its own traversal would test.
+// A path that hits nothing ends here with the background's radiance; the
+// others write their state and join the first queue. (Batch of 32 scenes, 74.4
+// million paths of which 9 in 10 hit nothing: 27.4 -> 21.9 ms with this and
+// the list of shadow work that shade keeps; the sphere cloud's frame, whose
+// camera rays were written, read and shaded whether they hit or not, 24.44 ->
+// 24.11.)
 template <bool COUNT, bool ONE>
-__global__ void __launch_bounds__(kWfMaxBlock) wf_extend_packet(WfArgs A) {
+__global__ void __launch_bounds__(kWfMaxBlock) wf_camera(WfArgs A, long long path_begin, int n_slots) {
     __shared__ int s_ref[kWfMaxBlock / 32][kMaxStack];
     __shared__ float s_key[kWfMaxBlock / 32][kMaxStack];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int* sref = s_ref[warp];
     float* skey = s_key[warp];
     RayCount rc = {};
-    const QView qv = qview(A, 0);
     unsigned int* cursor = A.work + 0;
     while (true) {
         const int base = fetch32(cursor);
-        if (base >= qv.total) break;
-        const int e = base + lane;
-        const bool valid = e < qv.total;
-        const int slot = valid ? qv.slot(e) : -1;
-        int view = 0;
-        if constexpr (!ONE) {
-            view = valid ? A.jobs[A.st[slot].w].view : -1;
-            const int view0 = __shfl_sync(0xffffffffu, view, 0);   // lane 0 has a ray
-            if (!__all_sync(0xffffffffu, !valid || view == view0)) {
-                if (valid) {
-                    const SceneView& Sv = A.views[view];
-                    const float4 o = A.ray_o[slot], d = A.ray_d[slot];
-                    if (COUNT) rc.ext++;
-                    ClosestTrav4<0, COUNT> t1;
-                    TravStack<0> st1;
-                    if (!t1.init(Sv, Ray{v3(o.x, o.y, o.z), v3(d.x, d.y, d.z)}, 1e-4f, 1e9f,
-                                 &rc.tc))
-                        while (!t1.step(Sv, st1, &rc.tc)) {
-                        }
-                    A.hit[slot] = make_float4(t1.t_best, __int_as_float(t1.best_ref),
-                                              __int_as_float(t1.best), 0.0f);
-                }
-                continue;
-            }
-            view = view0;
-        }
-        const SceneView& S = ONE ? A.view0 : A.views[view];
-        ClosestTrav4<kWfShared, COUNT> tr;
-        bool active = false;
+        if (base >= n_slots) break;
+        const int slot = base + lane;
+        const bool valid = slot < n_slots;
+        const int jb = ONE || !valid ? 0 : find_job(A.jobs, A.n_jobs, path_begin + slot);
+        const SceneView& Sv = view_of<ONE>(A, jb);
+        CameraPath cp{};
+        bool live = false;
         if (valid) {
-            const float4 o = A.ray_o[slot], d = A.ray_d[slot];
-            if (COUNT) rc.ext++;
-            active = !tr.init(S, Ray{v3(o.x, o.y, o.z), v3(d.x, d.y, d.z)}, 1e-4f, 1e9f, &rc.tc);
+            cp = camera_path(job_of<ONE>(A, jb), Sv, path_begin + slot);
+            if (COUNT) rc.ref++;
+            live = job_of<ONE>(A, jb).P.depth > 0;
+            if (COUNT && live) rc.ext++;
         }
+        ClosestTrav4<kWfShared, COUNT> tr;
+        tr.best = -1;
+        bool active = live && !tr.init(Sv, cp.ray, 1e-4f, 1e9f, &rc.tc);
+        // the packet's scene: that of its first ray still in the air
+        const unsigned air = __ballot_sync(0xffffffffu, active);
+        const SceneView* Sp = &Sv;
+        if constexpr (!ONE) {
+            const int first = air ? __ffs(air) - 1 : 0;
+            const int view = A.jobs[jb].view, view0 = __shfl_sync(0xffffffffu, view, first);
+            if (!__all_sync(0xffffffffu, !active || view == view0)) {
+                if (active) {
+                    TravStack<0> st1;
+                    ClosestTrav4<0, COUNT> t1;
+                    t1.init(Sv, cp.ray, 1e-4f, 1e9f, nullptr);
+                    while (!t1.step(Sv, st1, &rc.tc)) {
+                    }
+                    tr.t_best = t1.t_best;
+                    tr.best_ref = t1.best_ref;
+                    tr.best = t1.best;
+                }
+                active = false;
+            }
+            Sp = &A.views[view0];
+        }
+        const SceneView& S = *Sp;
         // lanes without a ray still load each node the packet enters: give
         // them the lo-first plane order
         if (!active) tr.rp.ox = tr.rp.oy = tr.rp.oz = 0;
@@ -506,9 +537,23 @@ __global__ void __launch_bounds__(kWfMaxBlock) wf_extend_packet(WfArgs A) {
                 if (!found) break;
             }
         }
-        if (valid)
+        // the hits go on, the others end with the background (a path that is
+        // never traced, of depth 0, with nothing)
+        const bool hit = live && tr.best >= 0;
+        if (hit) {
+            A.ray_o[slot] = make_float4(cp.ray.o.x, cp.ray.o.y, cp.ray.o.z, 0.0f);
+            A.ray_d[slot] = make_float4(cp.ray.d.x, cp.ray.d.y, cp.ray.d.z, 0.0f);
             A.hit[slot] = make_float4(tr.t_best, __int_as_float(tr.best_ref),
                                       __int_as_float(tr.best), 0.0f);
+            const PathParams& P = job_of<ONE>(A, jb).P;
+            A.st[slot] = make_uint4(cp.rng.s, (unsigned)P.depth,
+                                    P.mode == kModeWhitted ? kFlagWhitted : 0u, (unsigned)jb);
+        } else if (valid) {
+            V3 L = v3(0, 0, 0);
+            if (live) L = L + v3(1.0f, 1.0f, 1.0f) * ld3(Sv.bg);
+            A.L[slot] = make_float4(L.x, L.y, L.z, 0.0f);
+        }
+        warp_append(hit, slot, A.counts, A.q[0], lane);
     }
     flush_counts<COUNT>(A, rc, 1);
 }
@@ -614,10 +659,12 @@ wf_shade(WfArgs A, int it) {
                 if (A.sort_key == 3) key_next = sort_key_of<kMortonBitsE>(S, ps.ray.o, ps.ray.d);
             }
         }
-        // sort key 2: the unsorted list of slots with shadow work and their
-        // keys, ordered by wf_sort_scatter
+        // the list of slots with shadow work; sort key 2: with their keys,
+        // ordered by wf_sort_scatter
+        if (A.sort_key >= 2 || A.shadow_list)
+            warp_append(shadow_work, slot, A.tcnt + 2 * it + 1, A.tmp_s, lane,
+                        A.sort_key >= 2 ? A.key_s : nullptr, key);
         if (A.sort_key >= 2) {
-            warp_append(shadow_work, slot, A.tcnt + 2 * it + 1, A.tmp_s, lane, A.key_s, key);
             // bin counts, one atomic per distinct key in the warp
             const unsigned same = __match_any_sync(0xffffffffu, key);
             if (shadow_work && lane == __ffs(same) - 1) atomicAdd(A.hist_s + key, __popc(same));
@@ -758,9 +805,10 @@ wf_shadow(WfArgs A, int it) {
     stk.stride = blockDim.x;
     RayCount rc = {};
     const QView qv = qview(A, it);
-    // sort key 2: the slots with shadow work, sorted by their first shadow ray
-    const bool sorted = A.sort_key >= 2;
-    const int total = sorted ? A.tcnt[2 * it + 1] : qv.total;
+    // the slots with shadow work (sort key 2: sorted by their first shadow
+    // ray), or the whole queue
+    const int* list = A.sort_key >= 2 ? A.qs : A.shadow_list ? A.tmp_s : nullptr;
+    const int total = list ? A.tcnt[2 * it + 1] : qv.total;
     unsigned int* cursor = A.work + it * 3 + 2;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
@@ -821,7 +869,7 @@ wf_shadow(WfArgs A, int it) {
             if (!active) {
                 const int e = base + __popc(idle & below);
                 if (e < total) {
-                    slot = sorted ? A.qs[e] : qv.slot(e);
+                    slot = list ? list[e] : qv.slot(e);
                     const int info = __float_as_int(A.rec[(size_t)slot * 4 + 3].w);
                     const int kind = info & 3;
                     if (kind != 0) {
@@ -1064,7 +1112,7 @@ static cudaError_t occupancy(WfOccupancy& o, int blk = kWfBlock) {
     o.grid_accumulate = sms * 16 * kWfBlock / blk;
     int b4 = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b4, wf_extend_packet<COUNT, ONE>, blk, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b4, wf_camera<COUNT, ONE>, blk, 0);
     o.grid_packet = sms * std::max(b4, 1);
     return e;
 }
@@ -1135,14 +1183,16 @@ static cudaError_t enqueue_frame(const WfScratch& W, const std::vector<WfJob>& j
         size_t cnt_bytes = (size_t)(iters + 2) * kOctants * 4;
         if ((e = cudaMemsetAsync(A.counts, 0, cnt_bytes, st)) != cudaSuccess) return e;
         if ((e = cudaMemsetAsync(A.work, 0, (size_t)(iters + 2) * 3 * 4, st)) != cudaSuccess) return e;
-        if (A.sort_key >= 2 &&
-            (e = cudaMemsetAsync(A.tcnt, 0, (size_t)(iters + 2) * 2 * 4, st)) != cudaSuccess)
+        if ((e = cudaMemsetAsync(A.tcnt, 0, (size_t)(iters + 2) * 2 * 4, st)) != cudaSuccess)
             return e;
-        int gblocks = (int)((slots + blk - 1) / blk);
-        lt.mark(KC_GENERATE, st, true);
-        wf_generate<COUNT, ONE><<<gblocks, blk, 0, st>>>(A, path_begin, (int)slots);
-        lt.mark(KC_GENERATE, st, false);
-        n_launch += 1;
+        const bool packets = packet_first && iters > 0;
+        if (!packets) {
+            const int gblocks = (int)((slots + blk - 1) / blk);
+            lt.mark(KC_GENERATE, st, true);
+            wf_generate<COUNT, ONE><<<gblocks, blk, 0, st>>>(A, path_begin, (int)slots);
+            lt.mark(KC_GENERATE, st, false);
+            n_launch += 1;
+        }
         // With a side stream, shadow k runs on it beside extend k+1 (they
         // touch disjoint state: shadow k reads the shadow records and pending
         // terms and adds to L, extend k+1 reads rays and writes hits); shade
@@ -1153,8 +1203,8 @@ static cudaError_t enqueue_frame(const WfScratch& W, const std::vector<WfJob>& j
         // three spheres, 19,200 paths: 0.20 -> 0.18).
         auto launch_extend = [&](int it) {
             lt.mark(KC_EXTEND, st, true);
-            if (it == 0 && packet_first)
-                wf_extend_packet<COUNT, ONE><<<occ.grid_packet, blk, 0, st>>>(A);
+            if (it == 0 && packets)
+                wf_camera<COUNT, ONE><<<occ.grid_packet, blk, 0, st>>>(A, path_begin, (int)slots);
             else
                 wf_extend<COUNT, ONE><<<occ.grid_extend, blk, smem, st>>>(A, it);
             lt.mark(KC_EXTEND, st, false);
@@ -1278,6 +1328,7 @@ cudaError_t wavefront_render(WfScratch& W, const std::vector<SceneView>& views,
     W.args.packets = packets ? 1 : 0;
     W.args.refill_below = refill > 0 ? refill : kDefaultRefill;
     W.args.maxS = maxS;
+    W.args.shadow_list = maxS <= 2 ? 1 : 0;
     W.block = block > 0 ? block : kWfBlock;
     const bool one = n == 1;
     if (one) {
