@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -69,6 +70,8 @@ struct DeviceScene {
     int depth = 0;
     int n_materials = 0;
     bool has_glass = false;            // a dielectric material (two-branch glass needs it)
+    bool has_reflective = false;       // a material that continues a Whitted path
+    bool has_long_kinds = false;       // cubes, cylinders or cones
     std::vector<DevLight> lights;
     std::vector<int> quad_mats;        // material ids of quad-light emitters
     DevMaterial* d_mats = nullptr;
@@ -925,9 +928,16 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
             return cuda_fail(c, e, "scene upload");
         }
     }
-    // the glass flag while the copies run
+    // the material and primitive kinds while the copies run
     const bool has_glass = first_bad(s->n_materials, [&](int k) {
         return s->materials[k].kind == PGPU_MAT_DIELECTRIC;
+    }) >= 0;
+    const bool has_reflective = has_glass || first_bad(s->n_materials, [&](int k) {
+        return s->materials[k].kind == PGPU_MAT_METAL;
+    }) >= 0;
+    const bool has_long_kinds = first_bad(s->n_prims, [&](int k) {
+        const int t = s->prims[k].type;
+        return t == PGPU_PRIM_CUBE || t == PGPU_PRIM_CYLINDER || t == PGPU_PRIM_CONE;
     }) >= 0;
     e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
@@ -967,6 +977,8 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     ds->depth = depth;
     ds->n_materials = s->n_materials;
     ds->has_glass = has_glass;
+    ds->has_reflective = has_reflective;
+    ds->has_long_kinds = has_long_kinds;
     ds->lights = std::move(lights);
     ds->quad_mats = std::move(quad_mats);
     ds->d_mats = reinterpret_cast<DevMaterial*>(base + off_mt);
@@ -1055,18 +1067,20 @@ int32_t pgpu_update_materials(pgpu_ctx* c, int32_t id, const pgpu_material* m, i
     if (!m || n != ds->n_materials)
         return fail(c, PGPU_ERR_INVALID_ARG, "material count %d, scene has %d", n, ds->n_materials);
     std::vector<DevMaterial> mats(n);
-    bool has_glass = false;
+    bool has_glass = false, has_reflective = false;
     for (int k = 0; k < n; ++k) {
         if (m[k].kind < PGPU_MAT_DIFFUSE || m[k].kind > PGPU_MAT_DIELECTRIC || m[k].flags != 0)
             return fail(c, PGPU_ERR_UNSUPPORTED, "material %d unsupported", k);
         mats[k] = dev_material(m[k]);
         has_glass = has_glass || m[k].kind == PGPU_MAT_DIELECTRIC;
+        has_reflective = has_reflective || m[k].kind != PGPU_MAT_DIFFUSE;
     }
     for (int q : ds->quad_mats) mats[q].area_emitter = 1;
     PGPU_CUDA(c, cudaMemcpyAsync(ds->d_mats, mats.data(), mats.size() * sizeof(DevMaterial),
                                  cudaMemcpyHostToDevice, c->stream));
     PGPU_CUDA(c, cudaStreamSynchronize(c->stream));
     ds->has_glass = has_glass;
+    ds->has_reflective = has_reflective;
     return PGPU_OK;
 }
 
@@ -1163,6 +1177,40 @@ int run_wavefront(pgpu_ctx* c, const std::vector<DeviceScene*>& scenes,
     return PGPU_OK;
 }
 
+// Whether a frame of the wavefront engine runs as one kernel, a thread per
+// path (mk_render, which makes the same image bit for bit), instead of the
+// queued kernels. Queues pay three kernels a bounce, each as long as its
+// longest ray; one kernel pays once, but its warps run their paths' parts in
+// turn, which costs more the more rays there are and the more they diverge.
+// So the line is drawn by the rays of a first vertex, and by what makes them
+// diverge: the depth of the tree and the kinds of primitives. Queued / one
+// kernel, ms, by paths:
+//   path tracing, one light, up to 1024 leaves: 4 leaves 0.33 / 0.19 (528k),
+//     0.45 / 0.46 (1.1M); 300 leaves 0.30 / 0.12 (528k); three lights, 62
+//     triangles 0.59 / 0.40 (128k), 0.91 / 1.13 (528k)
+//   more leaves: 5,000 spheres 0.42 / 0.26 (128k), 0.55 / 0.56 (528k); 100,000
+//     spheres 1.32 / 0.99 (64k), 1.47 / 1.49 (128k); 5,000 triangles 0.82 /
+//     0.81 (128k); 328,000 triangles 1.51 / 1.05 (128k)
+//   cubes, cylinders or cones, three lights: 63 leaves 1.00 / 0.83 (64k), 1.10
+//     / 1.49 (128k); 253 leaves 1.59 / 1.40 (24k), 1.92 / 2.67 (64k)
+//   Whitted mode, where only glass and metal continue: 63 leaves 1.08 / 0.43
+//     (230k), 10.5 / 7.4 (14.7M); 328,000 triangles without glass or metal
+//     14.8 / 10.6 (14.7M); 303 leaves 2.6 / 1.6 (230k), 4.0 / 4.7 (1.2M);
+//     20,000 spheres 0.61 / 0.50 (230k), 1.06 / 1.63 (1.2M)
+// Frames that count, profile or set a launch parameter keep the queues.
+static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
+    if (c.count || c.profile || !c.packets || c.queue_capacity || c.sort_key || c.refill ||
+        c.block || std::getenv("PGPU_INJECT_SHADOW_RECORDS"))
+        return false;
+    const long long paths = c.pixels() * c.spp;
+    if (c.mode == PGPU_MODE_WHITTED)
+        return ds.n_leaves <= 256 || !ds.has_reflective || paths <= (1 << 18);
+    long long rays = 1;                 // of a path-traced vertex
+    for (const DevLight& l : ds.lights) rays += l.is_emissive ? 0 : 1;
+    const long long most = ds.has_long_kinds ? 1 << 17 : ds.n_leaves <= 1024 ? 1 << 20 : 1 << 18;
+    return paths * rays <= most;
+}
+
 // pgpu_render and pgpu_render_window: the image, or the window `win` of it.
 static int32_t render_impl(pgpu_ctx* c, int32_t id, const pgpu_render_params* p,
                            const int32_t* win, float* out_rgb, float* out_m2, pgpu_stats* stats) {
@@ -1201,7 +1249,8 @@ static int32_t render_impl(pgpu_ctx* c, int32_t id, const pgpu_render_params* p,
     double kms[KC_N] = {0};
     PGPU_CUDA(c, cudaEventRecord(c->ev0, c->stream));
     cudaError_t e;
-    if (cfg.engine == PGPU_ENGINE_MEGAKERNEL) {
+    if (cfg.engine == PGPU_ENGINE_MEGAKERNEL || one_kernel_frame(*ds, cfg)) {
+        *c->h_status = 0;
         e = launch_megakernel(ds->view, cfg, d_out, d_m2, c->d_cnt, c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "megakernel launch");
     } else {

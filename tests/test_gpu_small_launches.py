@@ -51,3 +51,63 @@ def test_more_shadow_rays_than_lanes(gpu, soft, binary_tree):
         b = gpu.render(sid, dataclasses.replace(st, count_rays=True))
         assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     gpu.free(sid)
+
+
+# frames that run as one kernel unless a launch parameter asks for the queues
+@pytest.mark.parametrize("name", ["three_spheres", "prims_mix", "cloud2k", "mesh_small", "shapes"])
+@pytest.mark.parametrize("pathtrace", [False, True])
+def test_queues_render_what_one_kernel_renders(gpu, name, pathtrace):
+    """Every launch parameter that keeps a small frame on the queued kernels:
+    camera packets that end their misses and compact their hits, camera rays
+    one per lane, chunks, every sort key. Ragged sizes; second moments too."""
+    scene, _ = load_golden(name)
+    sid = gpu.upload(scene)
+    for w, h, n in ((1, 1, 1), (7, 5, 2), (61, 47, 3)):
+        st = RenderSettings(width=w, height=h, samples=n, max_depth=5, pathtrace=pathtrace,
+                            pathtrace_bounces=5, seed=3)
+        m2 = np.empty((h, w, 3), np.float32)
+        ref = gpu.render(sid, st, None, m2)
+        for kw in (dict(block_size=128), dict(packets=False), dict(queue_capacity=64),
+                   dict(sort_key=1), dict(sort_key=2), dict(sort_key=3), dict(refill_below=1)):
+            q2 = np.empty_like(m2)
+            img = gpu.render(sid, dataclasses.replace(st, **kw), None, q2)
+            assert np.array_equal(img.view(np.uint32), ref.view(np.uint32)), kw
+            assert np.array_equal(q2.view(np.uint32), m2.view(np.uint32)), kw
+    gpu.free(sid)
+
+
+def test_batch_of_scenes_that_hit_and_miss(gpu):
+    """Camera packets over jobs of different scenes, among them one whose
+    camera sees nothing, one without primitives' light and one of depth 0."""
+    from pencil_b200.scene import CameraArgs, Scene
+    scene, _ = load_golden("cloud2k")
+    empty = Scene()
+    empty.background = (0.2, 0.3, 0.4)
+    away = CameraArgs((0, 0, -120), (0, 0, -240), (0, 1, 0), 45.0, 1.0)
+    sids = [gpu.upload(scene), gpu.upload(empty), gpu.upload(scene, None, away),
+            gpu.upload(scene)]
+    sts = [RenderSettings(width=w, height=h, samples=n, pathtrace=True, pathtrace_bounces=d)
+           for w, h, n, d in ((33, 9, 1, 4), (5, 7, 2, 3), (11, 3, 3, 4), (6, 5, 1, 0))]
+    outs = gpu.render_batch(sids, sts)
+    for sid, st, out in zip(sids, sts, outs):
+        one = gpu.render(sid, dataclasses.replace(st, packets=False))
+        assert np.array_equal(out.view(np.uint32), one.view(np.uint32))
+    assert np.all(outs[1] == np.array(empty.background, np.float32))
+    assert not outs[3].any()
+    for sid in sids:
+        gpu.free(sid)
+
+
+@pytest.mark.parametrize("side", [0, 1])
+def test_both_sides_of_the_one_kernel_line(gpu, side):
+    """A frame on the line (2^20 rays of first vertices in a small scene) and
+    the next larger one: the same pixels where they are the same."""
+    scene, _ = load_golden("three_spheres")
+    sid = gpu.upload(scene)
+    rays = 1 + sum(not l.is_emissive for l in scene.lights)
+    st = RenderSettings(width=64, height=(1 << 20) // rays // 64 + side, samples=1,
+                        pathtrace=True, pathtrace_bounces=3)
+    a = gpu.render(sid, st)
+    b = gpu.render(sid, dataclasses.replace(st, block_size=128))
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    gpu.free(sid)
