@@ -299,6 +299,8 @@ struct DevBuf {
 //   children   the two ranges, their boxes (the prefix / suffix merges, equal
 //              to the merge of their primitives' boxes) and their DFS
 //              pre-order indices (a subtree over c primitives has 2c - 1 nodes)
+// A node of up to kSahLocal primitives leaves these passes: one block builds
+// its whole subtree in shared memory (sah_local).
 // Nodes of 2 to 4 primitives finish in one thread each with Pencil's median
 // split (sort by centroid sum, split at the middle) down to the leaves; a
 // larger node whose axis has no extent, or whose primitives all fall in one
@@ -306,6 +308,11 @@ struct DevBuf {
 constexpr int kSahBuckets = 12;
 constexpr int kSahChunk = 1024;    // primitives per block of the bin / partition passes
 constexpr int kSahBlock = 256;
+// Primitives of a subtree that one block builds alone. A level of the passes
+// is eleven launches and a round trip to the host whatever it holds, and the
+// lower half of a tree's levels holds only small nodes; their median splits
+// went through a segmented sort of three more launches.
+constexpr int kSahLocal = 512;
 // The quality variant (traversal trees, not Pencil's tree): buckets over the
 // node's centroid bounds rather than its box, on all three axes.
 constexpr int kQualBuckets = 16;
@@ -378,9 +385,13 @@ __device__ __forceinline__ int item_task(const int* item_off, int T, int item) {
     return lo;
 }
 
-__global__ void sah_chunks(const SahTask* tasks, int T, int* nchunk) {
+// `T` bounds the level's task count *n_tasks (the host learns the count only
+// with the level's results); the slots beyond it have no chunks, and so no
+// items in the passes over items.
+__global__ void sah_chunks(const SahTask* tasks, const int* n_tasks, int T, int* nchunk) {
+    const int n = *n_tasks;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x)
-        nchunk[t] = (tasks[t].count + kSahChunk - 1) / kSahChunk;
+        nchunk[t] = t < n ? (tasks[t].count + kSahChunk - 1) / kSahChunk : 0;
 }
 
 __global__ void sah_bins_init(SahBin* bins, int n) {
@@ -542,9 +553,10 @@ __device__ __forceinline__ void sah_best_boundary(const SahBin* b, int nb, int a
 // the quality variant, the best boundary over the three axes' bins -- or the
 // median split along the box's longest axis when no boundary separates.
 template <bool Q>
-__global__ void sah_choose(const SahTask* tasks, int T, const SahBin* bins, const int* cb,
-                           SahChoice* ch, int* fb_list, int* n_fb) {
+__global__ void sah_choose(const SahTask* tasks, const int* n_tasks, const SahBin* bins,
+                           const int* cb, SahChoice* ch, int* fb_list, int* n_fb) {
     constexpr int NB = kBinsPerTask<Q>;
+    const int T = *n_tasks;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
         const SahTask tk = tasks[t];
         SahChoice c;
@@ -734,9 +746,11 @@ __device__ __forceinline__ void sah_write(pgpu_bvh_node* nodes, int total, int a
 
 // One thread per task: the node's row, and its two children -- a leaf, a
 // small task (2 to 4 primitives) or a task of the next level.
-__global__ void sah_children(const SahTask* tasks, int T, const SahChoice* ch, const int* perm,
-                             SahTask* next, int* n_next, SahSmall* small, int* n_small,
+__global__ void sah_children(const SahTask* tasks, const int* n_tasks, const SahChoice* ch,
+                             const int* perm, SahTask* next, int* n_next, int local_max,
+                             SahTask* local, int* n_local, SahSmall* small, int* n_small,
                              pgpu_bvh_node* nodes, int total, int* max_level) {
+    const int T = *n_tasks;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
         const SahTask tk = tasks[t];
         const SahChoice c = ch[t];
@@ -761,9 +775,191 @@ __global__ void sah_children(const SahTask* tasks, int T, const SahChoice* ch, c
                 nt.node = node;
                 nt.level = tk.level + 1;
                 for (int a = 0; a < 3; ++a) { nt.mn[a] = mn[a]; nt.mx[a] = mx[a]; }
-                next[atomicAdd(n_next, 1)] = nt;
+                if (cnt <= local_max) local[atomicAdd(n_local, 1)] = nt;
+                else next[atomicAdd(n_next, 1)] = nt;
             }
         }
+    }
+}
+
+// One block per subtree of 5 to kSahLocal primitives: sah_bin, sah_choose, the
+// stable partition or median split and sah_children for every node of it with
+// more than 4 primitives, a warp per node, level by level. The primitives'
+// boxes and their order stay in shared memory; the order goes back to `perm`
+// for sah_small. What bounds it is the latency of a node's steps, a few
+// microseconds each, over the subtree's ten levels or so.
+__global__ void __launch_bounds__(kSahBlock)
+sah_local(const SahTask* local, const int* n_local, int* perm, const DBox* boxes,
+          SahSmall* small, int* n_small, pgpu_bvh_node* nodes, int total, int* max_level) {
+    constexpr int kWarps = kSahBlock / 32;
+    constexpr int kTasks = kSahLocal / 5 + 1;
+    __shared__ DBox s_box[kSahLocal];
+    __shared__ int s_prim[kSahLocal], s_perm[kSahLocal], s_tmp[kSahLocal];
+    __shared__ SahTask s_task[2][kTasks];
+    __shared__ int s_n[2];
+    __shared__ SahBin s_bin[kWarps][kSahBuckets];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u, all = 0xffffffffu;
+    for (int job = blockIdx.x; job < *n_local; job += gridDim.x) {
+        const SahTask root = local[job];
+        for (int i = threadIdx.x; i < root.count; i += blockDim.x) {
+            const int prim = perm[root.start + i];
+            s_prim[i] = prim;
+            s_perm[i] = i;
+            s_box[i] = boxes[prim];
+        }
+        if (threadIdx.x == 0) {
+            s_task[0][0] = root;
+            s_n[0] = 1;
+            s_n[1] = 0;
+        }
+        __syncthreads();
+        for (int cur = 0; s_n[cur] > 0; cur ^= 1) {
+            const int n = s_n[cur];
+            for (int k = warp; k < n; k += kWarps) {
+                const SahTask tk = s_task[cur][k];
+                const int off = tk.start - root.start, count = tk.count;
+                const int axis = sah_axis(tk.mn, tk.mx);
+                SahBin* bin = s_bin[warp];
+                float cost = FLT_MAX;
+                int nl = 0;
+                DBox lb, rb;            // of the split before this lane's bucket
+                for (int a = 0; a < 3; ++a) {
+                    lb.mn[a] = rb.mn[a] = 1e30f;
+                    lb.mx[a] = rb.mx[a] = -1e30f;
+                }
+                if (tk.mx[axis] > tk.mn[axis]) {
+                    if (lane < kSahBuckets) {
+                        SahBin b;
+                        b.count = 0;
+                        for (int a = 0; a < 3; ++a) { b.mn[a] = ord(1e30f); b.mx[a] = ord(-1e30f); }
+                        bin[lane] = b;
+                    }
+                    __syncwarp();
+                    for (int i = lane; i < count; i += 32) {
+                        const DBox& b = s_box[s_perm[off + i]];
+                        SahBin* g = bin + sah_bucket(b, axis, tk.mn[axis], tk.mx[axis]);
+                        atomicAdd(&g->count, 1);
+                        for (int a = 0; a < 3; ++a) {
+                            atomicMin(&g->mn[a], ord(b.mn[a]));
+                            atomicMax(&g->mx[a], ord(b.mx[a]));
+                        }
+                    }
+                    __syncwarp();
+                    // lane i: the boundary between buckets i - 1 and i
+                    if (lane >= 1 && lane < kSahBuckets) {
+                        for (int j = 0; j < kSahBuckets; ++j) {
+                            DBox& d = j < lane ? lb : rb;
+                            for (int a = 0; a < 3; ++a) {
+                                d.mn[a] = fminf(d.mn[a], unord(bin[j].mn[a]));
+                                d.mx[a] = fmaxf(d.mx[a], unord(bin[j].mx[a]));
+                            }
+                            if (j < lane) nl += bin[j].count;
+                        }
+                        const int nr = count - nl;
+                        if (nl > 0 && nr > 0) {
+                            const float sa_parent = sah_area(tk.mn, tk.mx);
+                            const float c = 1.0f + ((float)nl * sah_area(lb.mn, lb.mx) +
+                                                    (float)nr * sah_area(rb.mn, rb.mx)) /
+                                                       (sa_parent > 0 ? sa_parent : 1.0f);
+                            if (c < FLT_MAX) cost = c;
+                        }
+                    }
+                }
+                // the first of the cheapest boundaries (costs are at least 1)
+                const unsigned least = __reduce_min_sync(all, __float_as_uint(cost));
+                const bool split = __uint_as_float(least) < FLT_MAX;
+                if (split) {
+                    const int best = __ffs(__ballot_sync(all, __float_as_uint(cost) == least)) - 1;
+                    nl = __shfl_sync(all, nl, best);
+                    for (int a = 0; a < 3; ++a) {
+                        lb.mn[a] = __shfl_sync(all, lb.mn[a], best);
+                        lb.mx[a] = __shfl_sync(all, lb.mx[a], best);
+                        rb.mn[a] = __shfl_sync(all, rb.mn[a], best);
+                        rb.mx[a] = __shfl_sync(all, rb.mx[a], best);
+                    }
+                    int ln = 0, rn = 0;
+                    for (int i0 = 0; i0 < count; i0 += 32) {
+                        const bool on = i0 + lane < count;
+                        const int q = on ? s_perm[off + i0 + lane] : 0;
+                        const bool left = on && sah_bucket(s_box[q], axis, tk.mn[axis],
+                                                           tk.mx[axis]) < best;
+                        const unsigned lm = __ballot_sync(all, left);
+                        const unsigned rm = __ballot_sync(all, on && !left);
+                        if (on)
+                            s_tmp[off + (left ? ln + __popc(lm & below)
+                                              : nl + rn + __popc(rm & below))] = q;
+                        ln += __popc(lm);
+                        rn += __popc(rm);
+                    }
+                } else {
+                    // median split: each primitive's place in the stable order
+                    // by centroid sum
+                    nl = count / 2;
+                    for (int a = 0; a < 3; ++a) {
+                        lb.mn[a] = rb.mn[a] = 1e30f;
+                        lb.mx[a] = rb.mx[a] = -1e30f;
+                    }
+                    for (int i = lane; i < count; i += 32) {
+                        const int q = s_perm[off + i];
+                        const float key = sah_key2(s_box[q], axis);
+                        int rank = 0;
+                        for (int j = 0; j < count; ++j) {
+                            const float kj = sah_key2(s_box[s_perm[off + j]], axis);
+                            rank += (kj < key || (kj == key && j < i)) ? 1 : 0;
+                        }
+                        s_tmp[off + rank] = q;
+                        DBox& d = rank < nl ? lb : rb;
+                        for (int a = 0; a < 3; ++a) {
+                            d.mn[a] = fminf(d.mn[a], s_box[q].mn[a]);
+                            d.mx[a] = fmaxf(d.mx[a], s_box[q].mx[a]);
+                        }
+                    }
+                    for (int o = 16; o > 0; o >>= 1)
+                        for (int a = 0; a < 3; ++a) {
+                            lb.mn[a] = fminf(lb.mn[a], __shfl_xor_sync(all, lb.mn[a], o));
+                            lb.mx[a] = fmaxf(lb.mx[a], __shfl_xor_sync(all, lb.mx[a], o));
+                            rb.mn[a] = fminf(rb.mn[a], __shfl_xor_sync(all, rb.mn[a], o));
+                            rb.mx[a] = fmaxf(rb.mx[a], __shfl_xor_sync(all, rb.mx[a], o));
+                        }
+                }
+                __syncwarp();
+                for (int i = lane; i < count; i += 32) s_perm[off + i] = s_tmp[off + i];
+                __syncwarp();
+                if (lane < 2) {            // the node's row and its two children
+                    const int cnt = lane ? count - nl : nl;
+                    const int start = lane ? tk.start + nl : tk.start;
+                    const int node = lane ? tk.node + 2 * nl : tk.node + 1;
+                    const DBox& b = lane ? rb : lb;
+                    if (lane == 0)
+                        sah_write(nodes, total, tk.node, tk.mn, tk.mx, tk.node + 1,
+                                  tk.node + 2 * nl);
+                    if (cnt == 1) {
+                        sah_write(nodes, total, node, b.mn, b.mx, -1,
+                                  s_prim[s_perm[start - root.start]]);
+                        atomicMax(max_level, tk.level + 1);
+                    } else if (cnt <= 4) {
+                        small[atomicAdd(n_small, 1)] = SahSmall{start, cnt, node, tk.level + 1};
+                    } else {
+                        SahTask nt;
+                        nt.start = start;
+                        nt.count = cnt;
+                        nt.node = node;
+                        nt.level = tk.level + 1;
+                        for (int a = 0; a < 3; ++a) { nt.mn[a] = b.mn[a]; nt.mx[a] = b.mx[a]; }
+                        const int at = atomicAdd(&s_n[cur ^ 1], 1);
+                        if (at < kTasks) s_task[cur ^ 1][at] = nt;   // (nodes of a level are disjoint)
+                    }
+                }
+                __syncwarp();
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) s_n[cur] = 0;
+            __syncthreads();
+        }
+        for (int i = threadIdx.x; i < root.count; i += blockDim.x)
+            perm[root.start + i] = s_prim[s_perm[i]];
+        __syncthreads();
     }
 }
 
@@ -829,8 +1025,8 @@ __global__ void sah_root_box(const DBox* boxes, int n, int* bounds) {
         }
     }
 }
-__global__ void sah_root(const int* bounds, int n, SahTask* tasks, SahSmall* small,
-                         int* perm) {
+__global__ void sah_root(const int* bounds, int n, int local_max, SahTask* tasks, SahTask* local,
+                         SahSmall* small, int* perm) {
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x)
         perm[k] = k;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -840,7 +1036,7 @@ __global__ void sah_root(const int* bounds, int n, SahTask* tasks, SahSmall* sma
         t.node = 0;
         t.level = 1;
         for (int a = 0; a < 3; ++a) { t.mn[a] = unord(bounds[a]); t.mx[a] = unord(bounds[3 + a]); }
-        if (n > 4) tasks[0] = t;
+        if (n > 4) (n <= local_max ? local : tasks)[0] = t;
         else small[0] = SahSmall{0, n, 0, 1};
     }
 }
@@ -933,7 +1129,10 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
     const size_t np = (size_t)s.n_prims, nv = (size_t)s.n_mesh_vertices,
                  nt = (size_t)s.n_mesh_triangles;
     const size_t total = 2 * (size_t)n - 1;
-    const int t_max = n / 5 + 1;                          // tasks of > 4 primitives per level
+    // the largest subtree that sah_local builds (it builds Pencil's tree only)
+    const int local_max = Q ? 4 : kSahLocal;
+    const int t_max = n / (local_max + 1) + 1;            // tasks of more primitives per level
+    const int l_max = Q ? 1 : n / 5 + 1;                  // tasks of 5 to local_max, in all
     const int item_max = t_max + n / kSahChunk + 1;       // their chunks
     const int small_max = n / 2 + 1;                      // tasks of 2 to 4 primitives, in all
     auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
@@ -945,13 +1144,14 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
                                              n, t_max, (const int*)nullptr, (const int*)nullptr,
                                              0, 32, st);
     size_t bytes = al(np * sizeof(pgpu_prim)) + al(nv * 12) + al(nt * 12) +
-                   al((size_t)n * sizeof(DBox)) + 2 * al((size_t)n * 4) + al(8 * 4) +
+                   al((size_t)n * sizeof(DBox)) + 2 * al((size_t)n * 4) + al(10 * 4) +
                    2 * al((size_t)t_max * sizeof(SahTask)) + al((size_t)small_max * sizeof(SahSmall)) +
                    al((size_t)t_max * NB * sizeof(SahBin)) + al((size_t)t_max * 6 * 4) +
                    al((size_t)t_max * sizeof(SahChoice)) + 2 * al((size_t)t_max * 4) +
                    2 * al((size_t)item_max * 4) + 3 * al((size_t)t_max * 4) +
                    2 * al((size_t)n * 4) + 2 * al((size_t)n * 4) +
-                   al(total * sizeof(pgpu_bvh_node)) + al(scan_bytes) + al(seg_bytes) + al(2 * 4);
+                   al((size_t)l_max * sizeof(SahTask)) +
+                   al(total * sizeof(pgpu_bvh_node)) + al(scan_bytes) + al(seg_bytes) + al(4 * 4);
     DevBuf mem;
     cudaError_t e = mem.alloc(bytes, pool, st);
     if (e != cudaSuccess) return e;
@@ -963,7 +1163,7 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
     auto* d_boxes = reinterpret_cast<DBox*>(take((size_t)n * sizeof(DBox)));
     auto* d_perm = reinterpret_cast<int*>(take((size_t)n * 4));
     auto* d_tmp = reinterpret_cast<int*>(take((size_t)n * 4));
-    auto* d_ctr = reinterpret_cast<int*>(take(8 * 4));   // bounds[6], n_next, n_fb
+    auto* d_ctr = reinterpret_cast<int*>(take(10 * 4));  // bounds[6], n_fb, -, task counts[2]
     SahTask* d_task[2] = {reinterpret_cast<SahTask*>(take((size_t)t_max * sizeof(SahTask))),
                           reinterpret_cast<SahTask*>(take((size_t)t_max * sizeof(SahTask)))};
     auto* d_small = reinterpret_cast<SahSmall*>(take((size_t)small_max * sizeof(SahSmall)));
@@ -984,16 +1184,19 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
     auto* d_out = reinterpret_cast<pgpu_bvh_node*>(take(total * sizeof(pgpu_bvh_node)));
     void* d_scan_tmp = take(scan_bytes);
     void* d_seg_tmp = take(seg_bytes);
-    int* d_misc = reinterpret_cast<int*>(take(2 * 4));   // small tasks, deepest level
+    int* d_misc = reinterpret_cast<int*>(take(4 * 4));   // small tasks, deepest level, local tasks
+    auto* d_local = reinterpret_cast<SahTask*>(take((size_t)l_max * sizeof(SahTask)));
 
     if (np) e = cudaMemcpyAsync(d_prims, s.prims, np * sizeof(pgpu_prim), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && nv)
         e = cudaMemcpyAsync(d_verts, s.mesh_vertices, nv * 12, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && nt)
         e = cudaMemcpyAsync(d_idx, s.mesh_indices, nt * 12, cudaMemcpyHostToDevice, st);
-    const int init[8] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0, 0};
+    const int T0 = n > local_max ? 1 : 0;
+    const int init[10] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, 0, 0, T0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_ctr, init, sizeof(init), cudaMemcpyHostToDevice, st);
-    const int misc_init[2] = {n > 4 ? 0 : 1, 0};   // a root of 2 to 4 primitives is small
+    // a root of 2 to 4 primitives is small, one of up to local_max is local
+    const int misc_init[4] = {n > 4 ? 0 : 1, 0, n > 4 && n <= local_max ? 1 : 0, 0};
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_misc, misc_init, sizeof(misc_init), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
@@ -1003,15 +1206,19 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
     };
     lb_boxes<<<grid(n), B, 0, st>>>(d_prims, (int)np, d_verts, d_idx, (int)nt, d_boxes);
     sah_root_box<<<grid(n), B, 0, st>>>(d_boxes, n, d_ctr);
-    sah_root<<<grid(n), B, 0, st>>>(d_ctr, n, d_task[0], d_small, d_perm);
+    sah_root<<<grid(n), B, 0, st>>>(d_ctr, n, local_max, d_task[0], d_local, d_small, d_perm);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    int T = n > 4 ? 1 : 0;
+    // A level is launched for at most T tasks, twice those of the level above,
+    // and tells the host its task count with its median splits.
+    int T = T0;
     int cur = 0;
-    int host_ctr[2];
+    int host_ctr[4];
     // every level holds at least one node more than the previous: at most n levels
     for (int lvl = 0; T > 0 && lvl < n; ++lvl) {
         SahTask* tasks = d_task[cur];
-        sah_chunks<<<grid(T), B, 0, st>>>(tasks, T, d_nchunk);
+        const int* d_n = d_ctr + 8 + cur;
+        int* d_next = d_ctr + 8 + (cur ^ 1);
+        sah_chunks<<<grid(T), B, 0, st>>>(tasks, d_n, T, d_nchunk);
         if ((e = cub::DeviceScan::ExclusiveSum(d_scan_tmp, scan_bytes, d_nchunk, d_item_off, T,
                                                st)) != cudaSuccess)
             return e;
@@ -1024,8 +1231,9 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
         sah_bins_init<<<grid(T * NB), B, 0, st>>>(d_bins, T * NB);
         sah_bin<Q><<<grid_items, B, 0, st>>>(tasks, T, d_item_off, d_nchunk, d_perm, d_boxes,
                                              d_cb, d_bins);
-        if ((e = cudaMemsetAsync(d_ctr + 6, 0, 2 * 4, st)) != cudaSuccess) return e;
-        sah_choose<Q><<<grid(T), B, 0, st>>>(tasks, T, d_bins, d_cb, d_ch, d_fb, d_ctr + 7);
+        if ((e = cudaMemsetAsync(d_ctr + 6, 0, 4, st)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(d_next, 0, 4, st)) != cudaSuccess) return e;
+        sah_choose<Q><<<grid(T), B, 0, st>>>(tasks, d_n, d_bins, d_cb, d_ch, d_fb, d_ctr + 6);
         if ((e = cudaMemsetAsync(d_left_cnt, 0, (size_t)grid_items * 4, st)) != cudaSuccess)
             return e;
         sah_part_count<Q><<<grid_items, B, 0, st>>>(tasks, T, d_item_off, d_nchunk, d_ch, d_perm,
@@ -1039,11 +1247,12 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
                                                 d_perm);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         // median splits of this level
-        if ((e = cudaMemcpyAsync(host_ctr, d_ctr + 6, 2 * 4, cudaMemcpyDeviceToHost, st)) !=
+        if ((e = cudaMemcpyAsync(host_ctr, d_ctr + 6, 4 * 4, cudaMemcpyDeviceToHost, st)) !=
                 cudaSuccess ||
             (e = cudaStreamSynchronize(st)) != cudaSuccess)
             return e;
-        const int n_fb = host_ctr[1];
+        const int n_fb = host_ctr[0], n_tasks = host_ctr[2 + cur];
+        if (n_tasks == 0) break;
         if (n_fb > 0) {
             sah_fb_sizes<<<grid(n_fb), B, 0, st>>>(tasks, d_fb, n_fb, d_fb_size);
             if ((e = cub::DeviceScan::ExclusiveSum(d_scan_tmp, scan_bytes, d_fb_size, d_fb_off,
@@ -1071,15 +1280,17 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
             sah_fb_scatter<<<n_fb, B, 0, st>>>(tasks, d_ch, d_fb, d_fb_off, d_vals2, d_perm,
                                                d_boxes);
         }
-        sah_children<<<grid(T), B, 0, st>>>(tasks, T, d_ch, d_perm, d_task[cur ^ 1], d_ctr + 6,
-                                            d_small, d_misc, d_out, (int)total, d_misc + 1);
+        sah_children<<<grid(n_tasks), B, 0, st>>>(tasks, d_n, d_ch, d_perm, d_task[cur ^ 1],
+                                                  d_next, local_max, d_local, d_misc + 2, d_small,
+                                                  d_misc, d_out, (int)total, d_misc + 1);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(host_ctr, d_ctr + 6, 4, cudaMemcpyDeviceToHost, st)) !=
-                cudaSuccess ||
-            (e = cudaStreamSynchronize(st)) != cudaSuccess)
-            return e;
-        T = host_ctr[0];
+        T = std::min(2 * n_tasks, t_max);
         cur ^= 1;
+    }
+    if constexpr (!Q) {
+        sah_local<<<std::min(l_max, 148 * 4), kSahBlock, 0, st>>>(
+            d_local, d_misc + 2, d_perm, d_boxes, d_small, d_misc, d_out, (int)total, d_misc + 1);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if ((e = cudaMemcpyAsync(host_ctr, d_misc, 2 * 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
         (e = cudaStreamSynchronize(st)) != cudaSuccess)

@@ -186,3 +186,31 @@ def test_device_sah_edge_cases(gpu):
     s.add_plane((0, -1, 0), (0, 1, 0), m)       # a +-1e6 box: the root's bins all fall together
     nodes, depth = gpu.build_bvh_device(s, method="sah")
     assert check_table(nodes, s.n_unified) == depth
+
+
+@pytest.mark.parametrize("n", [5, 6, 31, 33, 511, 512, 513, 514, 1026, 1537, 5000])
+@pytest.mark.parametrize("kind", ["random", "grid", "line", "point", "lopsided"])
+def test_device_sah_subtrees_built_by_one_block(gpu, n, kind):
+    """Sizes around the subtrees that one block builds (512), with centres
+    that spread, tie, lie on a line, coincide (median splits only) or crowd
+    (deep trees): a valid table, and where no centre ties Pencil's tree node
+    for node."""
+    from pencil_b200.scene import Material, Scene
+    rng = np.random.default_rng(n)
+    c = rng.uniform(-10, 10, (n, 3)).astype(np.float32)
+    if kind == "grid":
+        c = np.round(c)
+    elif kind == "line":
+        c[:, 1:] = 0
+    elif kind == "point":
+        c[:] = c[0]
+    elif kind == "lopsided":
+        c = (np.sign(c) * np.abs(c / 10) ** 9 * 1e4).astype(np.float32)
+    s = Scene()
+    m = s.add_material(Material.diffuse((1, 1, 1)))
+    s.add_spheres(c, rng.uniform(0.01, 0.3, n).astype(np.float32), np.full(n, m, np.int32))
+    nodes, depth = gpu.build_bvh_device(s, "sah")
+    assert check_table(nodes, n) == depth
+    if kind == "random":
+        host, host_depth = s.build_bvh()
+        assert depth == host_depth and np.array_equal(nodes, host)
