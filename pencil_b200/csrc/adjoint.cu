@@ -5,7 +5,9 @@
 // counter-RNG seeds: the same camera rays, hits, next-event samples, Russian
 // roulette decisions and scatter directions as the production renderer
 // (shade_vertex in path.cuh; the control flow and random-number use below
-// follow it step for step), traced on the 4-wide tree the renderers walk
+// follow it step for step). Large frames take the paths' hits and their
+// lights' visibility from a pass of the wavefront kernels (wavefront_adjoint);
+// the others are traced here, on the 4-wide tree the renderers walk
 // (the same hits as Pencil's binary tree; at 80 registers, six blocks per
 // SM, 17.5 ms per gradient there against 19.8 ms on the binary tree -- at
 // 128 registers the binary tree had been the faster). No state of the
@@ -40,6 +42,16 @@ constexpr int kMaxTape = 16;        // vertices per path (depth <= 16)
 constexpr int kMaxAdjLights = 8;    // lights whose gradient a thread accumulates
 constexpr int kAdjBlock = 128;
 
+// What a wavefront pass over a chunk's paths found: per bounce and path of the
+// chunk the closest hit (t, ref, leaf slot) and a bit per shadow record, in
+// the order shade_vertex makes them, set where the light is visible.
+struct AdjFound {
+    const float4* hit;
+    const unsigned* vis;
+    size_t stride;         // entries per bounce
+    long long path_begin;  // the chunk's first path
+};
+
 struct AdjArgs {
     SceneView S;
     PathParams P;
@@ -50,6 +62,8 @@ struct AdjArgs {
     double* d_light;       // 3 per light
     float* out;            // forward image of the replayed samples (or null)
     unsigned long long* counters;
+    AdjFound found;
+    long long pix_begin, pix_end;   // pixels of this launch
 };
 
 // One path vertex on the tape. g (reflectivity times the Russian-roulette
@@ -86,16 +100,42 @@ __device__ __forceinline__ void flush_contrib(bool has, int key, V3 v, double* g
     }
 }
 
-template <bool COUNT>
+// FOUND: hits and visibility come from a wavefront pass instead of rays traced
+// here.
+template <bool COUNT, bool FOUND>
 struct Replay {
     const SceneView& S;
     const PathParams& P;
     TravStack<kAdjShared>& stk;
     RayCount& rc;
+    const AdjFound& found;
+    size_t at;             // FOUND: this path's entry of the current bounce
+    unsigned vis;          // FOUND: its shadow bits not used yet
 
-    __device__ __forceinline__ bool occluded(const Ray& r, float tmin, float tmax) {
+    __device__ __forceinline__ bool visible(const DevLight& l, const Ray& r, float tmin,
+                                            float tmax) {
+        if constexpr (FOUND) {
+            const bool v = vis & 1u;
+            vis >>= 1;
+            return v;
+        }
+        if (l.is_emissive) return true;
         if (COUNT) rc.shadow++;
-        return any_hit4<kAdjShared, COUNT>(S, r, tmin, tmax, stk, &rc.tc);
+        return !any_hit4<kAdjShared, COUNT>(S, r, tmin, tmax, stk, &rc.tc);
+    }
+    __device__ __forceinline__ int closest(const Ray& r, float& tb, int& bref) {
+        if constexpr (FOUND) {
+            const float4 h = __ldcs(found.hit + at);
+            vis = 0;
+            tb = h.x;
+            bref = __float_as_int(h.y);
+            const int slot = __float_as_int(h.z);
+            if (slot >= 0) vis = __ldcs(found.vis + at);
+            at += found.stride;
+            return slot;
+        }
+        if (COUNT) rc.ext++;
+        return closest_hit4<kAdjShared, COUNT>(S, r, 1e-4f, 1e9f, tb, bref, stk, &rc.tc);
     }
 
     // Replay one path; fills the tape (returns its length; each vertex with
@@ -114,10 +154,9 @@ struct Replay {
             tv.B = v3(0, 0, 0);
             tv.g = 0.0f;
             tv.emits = 0;
-            if (COUNT) rc.ext++;
             float tb;
             int bref;
-            int slot = closest_hit4<kAdjShared, COUNT>(S, r, 1e-4f, 1e9f, tb, bref, stk, &rc.tc);
+            const int slot = closest(r, tb, bref);
             if (slot < 0) {
                 tv.mat = -1;
                 tv.A = ld3(S.bg);
@@ -149,8 +188,7 @@ struct Replay {
                     float dist;
                     light_dir(l, h.p, rng, Ld, dist);
                     float ndotl = clampf(dot(h.n, Ld), 0.0f, 1.0f);
-                    bool vis = l.is_emissive || !occluded(Ray{sorg, Ld}, P.bias, dist - P.bias);
-                    if (!vis) continue;
+                    if (!visible(l, Ray{sorg, Ld}, P.bias, dist - P.bias)) continue;
                     tv.B = tv.B + ld3(l.intensity) * ndotl;
                     if (li < kMaxAdjLights) dlight[li] = dlight[li] + w * T * albedo * ndotl;
                 }
@@ -161,7 +199,7 @@ struct Replay {
                         V3 Ld;
                         float tmax, wq;
                         if (!quad_sample(l, h.p, h.n, sorg, P.bias, rng, Ld, tmax, wq)) continue;
-                        if (occluded(Ray{sorg, Ld}, P.bias, tmax)) continue;
+                        if (!visible(l, Ray{sorg, Ld}, P.bias, tmax)) continue;
                         tv.B = tv.B + ld3(l.intensity) * wq;
                         if (li < kMaxAdjLights) dlight[li] = dlight[li] + w * T * albedo * wq;
                     }
@@ -223,7 +261,7 @@ struct Replay {
                             float spec = powf(ndoth, m.shininess);
                             phong = ld3(m.specular_color) * (spec * m.specular);
                         }
-                        if (!l.is_emissive && occluded(Ray{sorg, Ld}, P.bias, dist - P.bias)) continue;
+                        if (!visible(l, Ray{sorg, Ld}, P.bias, dist - P.bias)) continue;
                         ca = ca + ld3(l.intensity) * ndotl;
                         ce = ce + ld3(l.intensity) * phong;
                         if (li < kMaxAdjLights)
@@ -276,22 +314,23 @@ struct Replay {
 // latency (per gradient: 16.45 ms; 17.49 at 80 registers, 16.70 at 64).
 constexpr int kAdjMinBlocks = 7;
 
-template <bool COUNT>
+template <bool COUNT, bool FOUND>
 __global__ void __launch_bounds__(kAdjBlock, kAdjMinBlocks)
 adjoint_kernel(AdjArgs A) {
     extern __shared__ int smem[];
     TravStack<kAdjShared> stk;
-    stk.sref = smem + threadIdx.x;
-    stk.st = reinterpret_cast<float*>(smem + kAdjShared * blockDim.x) + threadIdx.x;
-    stk.stride = blockDim.x;
+    if constexpr (!FOUND) {
+        stk.sref = smem + threadIdx.x;
+        stk.st = reinterpret_cast<float*>(smem + kAdjShared * blockDim.x) + threadIdx.x;
+        stk.stride = blockDim.x;
+    }
     RayCount rc = {};
     const PathParams& P = A.P;
-    Replay<COUNT> rp{A.S, P, stk, rc};
+    Replay<COUNT, FOUND> rp{A.S, P, stk, rc, A.found, 0, 0};
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long npix = (long long)P.W * P.H;
-    const long long pix = gid / A.G;
+    const long long pix = A.pix_begin + gid / A.G;
     const int lane_g = (int)(gid % A.G);
-    const bool active = pix < npix;
+    const bool active = pix < A.pix_end;
     TapeV tape[kMaxTape];
     V3 dlight[kMaxAdjLights];
     for (int k = 0; k < kMaxAdjLights; ++k) dlight[k] = v3(0, 0, 0);
@@ -313,6 +352,7 @@ adjoint_kernel(AdjArgs A) {
             float u, v;
             sample_uv(i, j, s % P.n, s / P.n, P.W, P.H, P.n, rng, u, v);
             V3 L;
+            if constexpr (FOUND) rp.at = (size_t)(pix * P.spp + s - A.found.path_begin);
             nt = rp.path(camera_ray(A.S.cam, u, v), rng, w, tape, dlight, L);
             acc = acc + L;
         }
@@ -381,10 +421,8 @@ adjoint_kernel(AdjArgs A) {
     }
 }
 
-cudaError_t launch_adjoint(const SceneView& S, const RenderCfg& c, const float* dl,
-                           double* d_albedo, double* d_emission, double* d_light, float* out,
-                           unsigned long long* counters, cudaStream_t st) {
-    AdjArgs A;
+static AdjArgs adjoint_args(const SceneView& S, const RenderCfg& c, const AdjointOut& o) {
+    AdjArgs A{};
     A.S = S;
     A.P = PathParams{c.W, c.H, c.n, c.spp, c.depth, c.mode, c.rng, c.glass, c.soft, c.bias,
                      c.salt, c.sample_offset, 0};
@@ -392,17 +430,38 @@ cudaError_t launch_adjoint(const SceneView& S, const RenderCfg& c, const float* 
     int lim = c.spp < 32 ? c.spp : 32;
     while (G * 2 <= lim) G *= 2;
     A.G = G;
-    A.dl = dl;
-    A.d_albedo = d_albedo;
-    A.d_emission = d_emission;
-    A.d_light = d_light;
-    A.out = out;
-    A.counters = counters;
-    long long threads = (long long)c.W * c.H * G;
-    unsigned blocks = (unsigned)((threads + kAdjBlock - 1) / kAdjBlock);
-    size_t smem = (size_t)kAdjShared * kAdjBlock * 8;
-    if (c.count) adjoint_kernel<true><<<blocks, kAdjBlock, smem, st>>>(A);
-    else adjoint_kernel<false><<<blocks, kAdjBlock, smem, st>>>(A);
+    A.dl = o.dl;
+    A.d_albedo = o.d_albedo;
+    A.d_emission = o.d_emission;
+    A.d_light = o.d_light;
+    A.out = o.image;
+    A.counters = o.counters;
+    return A;
+}
+
+static unsigned adjoint_blocks(const AdjArgs& A) {
+    return (unsigned)(((A.pix_end - A.pix_begin) * A.G + kAdjBlock - 1) / kAdjBlock);
+}
+
+cudaError_t launch_adjoint(const SceneView& S, const RenderCfg& c, const AdjointOut& o,
+                           cudaStream_t st) {
+    AdjArgs A = adjoint_args(S, c, o);
+    A.pix_end = (long long)c.W * c.H;
+    const size_t smem = (size_t)kAdjShared * kAdjBlock * 8;
+    const unsigned blocks = adjoint_blocks(A);
+    if (c.count) adjoint_kernel<true, false><<<blocks, kAdjBlock, smem, st>>>(A);
+    else adjoint_kernel<false, false><<<blocks, kAdjBlock, smem, st>>>(A);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_adjoint_found(const SceneView& S, const RenderCfg& c, const AdjointOut& o,
+                                 const float4* hit, const unsigned* vis, size_t stride,
+                                 long long pix_begin, long long pixels, cudaStream_t st) {
+    AdjArgs A = adjoint_args(S, c, o);
+    A.found = AdjFound{hit, vis, stride, pix_begin * c.spp};
+    A.pix_begin = pix_begin;
+    A.pix_end = pix_begin + pixels;
+    adjoint_kernel<false, true><<<adjoint_blocks(A), kAdjBlock, 0, st>>>(A);
     return cudaGetLastError();
 }
 

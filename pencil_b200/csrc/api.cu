@@ -41,9 +41,11 @@ cudaError_t wavefront_render_static(int device, const SceneView& view, const Dev
                                     float* m2, cudaStream_t st, int* status_host, int* launches,
                                     const char** why);
 size_t static_scratch_bytes();
-cudaError_t launch_adjoint(const SceneView& S, const RenderCfg& c, const float* dl,
-                           double* d_albedo, double* d_emission, double* d_light, float* out,
-                           unsigned long long* counters, cudaStream_t st);
+cudaError_t launch_adjoint(const SceneView& S, const RenderCfg& c, const AdjointOut& o,
+                           cudaStream_t st);
+cudaError_t wavefront_adjoint(WfScratch& W, const SceneView& view,
+                              const std::vector<DevLight>& lights, const RenderCfg& cfg,
+                              const AdjointOut& o, cudaStream_t st, int* launches, bool* done);
 int adjoint_max_depth();
 int adjoint_max_lights();
 cudaError_t launch_tonemap(const float* d_hdr, long long n_pixels, int mode, float exposure,
@@ -1465,8 +1467,12 @@ int32_t pgpu_adjoint(pgpu_ctx* c, int32_t id, const pgpu_render_params* p, const
     if (cfg.count)
         PGPU_CUDA(c, cudaMemsetAsync(c->d_cnt, 0, CNT_N * sizeof(unsigned long long), c->stream));
     PGPU_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    cudaError_t e = launch_adjoint(ds->view, cfg, d_dl, d_g, d_g + 3 * nm, d_g + 6 * nm,
-                                   out_rgb ? d_img : nullptr, c->d_cnt, c->stream);
+    const AdjointOut ao{d_dl, d_g, d_g + 3 * nm, d_g + 6 * nm, out_rgb ? d_img : nullptr, c->d_cnt};
+    int launches = 1;
+    bool done = false;
+    cudaError_t e = wavefront_adjoint(*c->wf, ds->view, ds->lights, cfg, ao, c->stream, &launches,
+                                      &done);
+    if (e == cudaSuccess && !done) e = launch_adjoint(ds->view, cfg, ao, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint launch");
     PGPU_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     if ((rc = wait_render(c))) return rc;
@@ -1491,7 +1497,7 @@ int32_t pgpu_adjoint(pgpu_ctx* c, int32_t id, const pgpu_render_params* p, const
         stats->extension_rays = cnt[CNT_EXT];
         stats->shadow_rays = cnt[CNT_SHADOW];
         stats->reference_rays = cnt[CNT_REF];
-        stats->kernel_launches = 1;
+        stats->kernel_launches = launches;
         stats->total_ms =
             std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }

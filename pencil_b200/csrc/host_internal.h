@@ -60,6 +60,17 @@ struct RenderCfg {
     long long pixels() const { return win[2] > 0 ? (long long)win[2] * win[3] : (long long)W * H; }
 };
 
+// Device buffers of an adjoint call: dLoss/dimage in; gradient sums (zeroed
+// before), the replayed samples' image (or null) and ray counters out.
+struct AdjointOut {
+    const float* dl;
+    double* d_albedo;
+    double* d_emission;
+    double* d_light;
+    float* image;
+    unsigned long long* counters;
+};
+
 // Device counters written by the kernels (atomic adds).
 enum DevCounter {
     CNT_EXT = 0,

@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
 #include <vector>
 
@@ -56,6 +57,9 @@ constexpr int kSortBins = 1 << (3 * kMortonBits + 3);
 // extension rays as well for a cheaper histogram and scan).
 constexpr int kMortonBitsE = 5;
 constexpr int kSortBinsE = 1 << (3 * kMortonBitsE + 3);
+// wavefront_adjoint: paths up to which one kernel is as fast, paths per chunk.
+constexpr long long kAdjOneKernel = 1 << 18;
+constexpr int kAdjChunk = 1 << 22;
 
 // One render job of the path space.
 struct WfJob {
@@ -81,6 +85,10 @@ struct WfArgs {
     float4* L;
     uint4* st;                // rng, depth, flags, job
     float4* hit;              // t, best ref, leaf slot, found
+    // the adjoint's pass (the KEEP instantiations) keeps every bounce's hits,
+    // bounce k's at k * keep of `hit`, and shadow results, a bit per record
+    size_t keep;
+    unsigned* vis;
     float4* pb;               // Whitted vertex: pending base.xyz, scale s
     float4* pw;               // Whitted vertex: pending weight.xyz
     // Shadow record k of a slot: one 64-byte block, [(k * Q + slot) * 4 + f],
@@ -164,6 +172,12 @@ __device__ __forceinline__ int sort_key_of(const SceneView& S, V3 o, V3 d) {
     const uint32_t m = spread_bits3(c[0]) | (spread_bits3(c[1]) << 1) | (spread_bits3(c[2]) << 2);
     const uint32_t oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
     return (int)((m << 3) | oct);
+}
+
+// The hits of bounce `it`. KEEP: the adjoint's pass.
+template <bool KEEP>
+__device__ __forceinline__ float4* hits_of(const WfArgs& A, int it) {
+    return KEEP ? A.hit + (size_t)it * A.keep : A.hit;
 }
 
 __device__ __forceinline__ int find_job(const WfJob* jobs, int n, long long path) {
@@ -320,7 +334,7 @@ wf_generate(WfArgs A, long long path_begin, int n_slots) {
 // between node steps; when few lanes of the warp are still busy, the idle
 // lanes take new rays from the queue (one atomic per warp), so warps keep
 // traversing instead of waiting for their slowest ray.
-template <bool COUNT, bool ONE>
+template <bool COUNT, bool ONE, bool KEEP>
 __global__ void __launch_bounds__(kWfMaxBlock)
 wf_extend(WfArgs A, int it) {
     extern __shared__ int smem[];
@@ -332,6 +346,7 @@ wf_extend(WfArgs A, int it) {
     const QView qv = qview(A, it);
     const bool sorted_e = A.sort_key == 3 && it > 0;   // shade sorted this queue too
     unsigned int* cursor = A.work + it * 3 + 0;
+    float4* const hits = hits_of<KEEP>(A, it);
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     ClosestTrav4<kWfShared, COUNT> tr;
@@ -360,7 +375,7 @@ wf_extend(WfArgs A, int it) {
                     if (COUNT) rc.ext++;
                     if (tr.init(scene(), Ray{v3(o.x, o.y, o.z), v3(d.x, d.y, d.z)}, 1e-4f, 1e9f,
                                 &rc.tc))
-                        A.hit[slot] = make_float4(tr.t_best, __int_as_float(tr.best_ref),
+                        hits[slot] = make_float4(tr.t_best, __int_as_float(tr.best_ref),
                                                   __int_as_float(tr.best), 0.0f);
                     else
                         active = true;
@@ -373,7 +388,7 @@ wf_extend(WfArgs A, int it) {
             continue;
         }
         if (active && tr.step(scene(), stk, &rc.tc)) {
-            A.hit[slot] = make_float4(tr.t_best, __int_as_float(tr.best_ref),
+            hits[slot] = make_float4(tr.t_best, __int_as_float(tr.best_ref),
                                       __int_as_float(tr.best), 0.0f);
             active = false;
         }
@@ -414,7 +429,7 @@ __device__ __forceinline__ void warp_append(bool take, int slot, int* counter, i
 // the list of shadow work that shade keeps; the sphere cloud's frame, whose
 // camera rays were written, read and shaded whether they hit or not, 24.44 ->
 // 24.11.)
-template <bool COUNT, bool ONE>
+template <bool COUNT, bool ONE, bool KEEP>
 __global__ void __launch_bounds__(kWfMaxBlock) wf_camera(WfArgs A, long long path_begin, int n_slots) {
     __shared__ int s_ref[kWfMaxBlock / 32][kMaxStack];
     __shared__ float s_key[kWfMaxBlock / 32][kMaxStack];
@@ -552,6 +567,7 @@ __global__ void __launch_bounds__(kWfMaxBlock) wf_camera(WfArgs A, long long pat
             V3 L = v3(0, 0, 0);
             if (live) L = L + v3(1.0f, 1.0f, 1.0f) * ld3(Sv.bg);
             A.L[slot] = make_float4(L.x, L.y, L.z, 0.0f);
+            if constexpr (KEEP) A.hit[slot] = make_float4(0.0f, 0.0f, __int_as_float(-1), 0.0f);
         }
         warp_append(hit, slot, A.counts, A.q[0], lane);
     }
@@ -602,7 +618,7 @@ struct StoreNee {
 
 // At most 72 registers (28 warps per SM): the shading state machine is
 // latency-bound, and the extra resident warps pay for a few spilled words.
-template <bool COUNT, bool ONE>
+template <bool COUNT, bool ONE, bool KEEP>
 __global__ void __maxnreg__(72)
 wf_shade(WfArgs A, int it) {
     RayCount rc = {};
@@ -629,7 +645,7 @@ wf_shade(WfArgs A, int it) {
             const float4 o = A.ray_o[slot], d = A.ray_d[slot];
             const float4 T = it == 0 ? make_float4(1.0f, 1.0f, 1.0f, 0.0f) : A.T[slot];
             const float4 L = it == 0 ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : A.L[slot];
-            float4 hv = A.hit[slot];
+            const float4 hv = hits_of<KEEP>(A, it)[slot];
             PathState ps;
             ps.ray = Ray{v3(o.x, o.y, o.z), v3(d.x, d.y, d.z)};
             ps.T = v3(T.x, T.y, T.z);
@@ -795,7 +811,7 @@ wf_sort_scatter(const int* list, const int* count, const int* keyof, int* hist,
 // blocks of 128 per SM -- too few warps to hide the latency of its loads.
 constexpr int kShadowMinBlocks = 3;
 
-template <bool COUNT, bool ONE>
+template <bool COUNT, bool ONE, bool KEEP>
 __global__ void __launch_bounds__(kWfMaxBlock, kShadowMinBlocks)
 wf_shadow(WfArgs A, int it) {
     extern __shared__ int smem[];
@@ -821,6 +837,7 @@ wf_shadow(WfArgs A, int it) {
     NeeAccum acc;
     V3 L = v3(0, 0, 0), c = v3(0, 0, 0);
     int slot = -1, k = 0, n = 0, group_end = 0;
+    unsigned vis = 0;                   // bit k: record k's light is visible
     bool active = false;
     bool exhausted = false;
 
@@ -840,8 +857,10 @@ wf_shadow(WfArgs A, int it) {
                              &rc.tc))
                     return true;
                 acc.add(L, c, group_end, !tr.hit);
+                if constexpr (KEEP) vis |= (tr.hit ? 0u : 1u) << (k & 31);
             } else {
                 acc.add(L, c, group_end, true);
+                if constexpr (KEEP) vis |= 1u << (k & 31);
             }
             ++k;
         }
@@ -854,6 +873,7 @@ wf_shadow(WfArgs A, int it) {
             sc = A.pb[slot].w;
         }
         acc.finish(L, v3(pt.x, pt.y, pt.z), w, sc);
+        if constexpr (KEEP) A.vis[(size_t)it * A.keep + slot] = vis;
         A.L[slot] = make_float4(L.x, L.y, L.z, 0.0f);
         return false;
     };
@@ -884,6 +904,7 @@ wf_shadow(WfArgs A, int it) {
                         L = v3(L4.x, L4.y, L4.z);
                         n = info >> 2;
                         k = 0;
+                        vis = 0;
                         active = advance();
                     }
                 }
@@ -896,6 +917,7 @@ wf_shadow(WfArgs A, int it) {
         }
         if (active && tr.step(scene(), stk, &rc.tc)) {
             acc.add(L, c, group_end, !tr.hit);
+            if constexpr (KEEP) vis |= (tr.hit ? 0u : 1u) << (k & 31);
             ++k;
             active = advance();
         }
@@ -1003,6 +1025,8 @@ struct WfScratch {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_shaded = nullptr;  // shade k and its sorts are done
     cudaEvent_t ev_shadow = nullptr;  // shadow k is done
+    void* kept = nullptr;             // the adjoint's hits and shadow results of every bounce
+    size_t kept_bytes = 0;
 };
 
 static size_t al(size_t x) { return (x + 255) & ~size_t(255); }
@@ -1090,21 +1114,23 @@ static int max_shadow_records(const SceneView& v, const std::vector<DevLight>& l
     return std::max(1, std::max(pt, wh));
 }
 
+static cudaError_t ensure_streams(WfScratch& W);
+
 struct WfOccupancy {
     int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_scatter = 0, grid_packet = 0;
     int grid_accumulate = 0;
 };
 
-template <bool COUNT, bool ONE>
+template <bool COUNT, bool ONE, bool KEEP = false>
 static cudaError_t occupancy(WfOccupancy& o, int blk = kWfBlock) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     size_t smem = (size_t)kWfShared * blk * 8;
     int b1 = 0, b2 = 0, b3 = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, wf_extend<COUNT, ONE>, blk, smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, wf_shade<COUNT, ONE>, blk, 0);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, wf_shadow<COUNT, ONE>, blk, smem);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, wf_extend<COUNT, ONE, KEEP>, blk, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, wf_shade<COUNT, ONE, KEEP>, blk, 0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b3, wf_shadow<COUNT, ONE, KEEP>, blk, smem);
     o.grid_extend = sms * std::max(b1, 1);
     o.grid_shade = sms * std::max(b2, 1);
     o.grid_shadow = sms * std::max(b3, 1);
@@ -1112,7 +1138,7 @@ static cudaError_t occupancy(WfOccupancy& o, int blk = kWfBlock) {
     o.grid_accumulate = sms * 16 * kWfBlock / blk;
     int b4 = 0;
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b4, wf_camera<COUNT, ONE>, blk, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b4, wf_camera<COUNT, ONE, KEEP>, blk, 0);
     o.grid_packet = sms * std::max(b4, 1);
     return e;
 }
@@ -1145,13 +1171,16 @@ struct LaunchTimer {
     }
 };
 
-// ONE: a one-scene frame (W.args.view0 / job0 hold its scene and job).
-template <bool COUNT, bool ONE>
-static cudaError_t enqueue_frame(const WfScratch& W, const std::vector<WfJob>& jobs, int iters,
-                                 int Qeff, cudaStream_t st, int* launches, LaunchTimer& lt) {
+// ONE: a one-scene frame (W.args.view0 / job0 hold its scene and job). Each
+// chunk of paths ends with its pixel sums, or with finish(first pixel, pixels).
+template <bool COUNT, bool ONE, bool KEEP = false>
+static cudaError_t enqueue_frame(
+    const WfScratch& W, const std::vector<WfJob>& jobs, int iters, int Qeff, cudaStream_t st,
+    int* launches, LaunchTimer& lt,
+    const std::function<cudaError_t(long long, long long)>* finish = nullptr) {
     const int blk = W.block;
     WfOccupancy occ;
-    cudaError_t e = occupancy<COUNT, ONE>(occ, blk);
+    cudaError_t e = occupancy<COUNT, ONE, KEEP>(occ, blk);
     if (e != cudaSuccess) return e;
     const bool packet_first = W.args.packets != 0;
     // timed (profiled) frames stay on one stream so that kernel classes add up
@@ -1204,9 +1233,9 @@ static cudaError_t enqueue_frame(const WfScratch& W, const std::vector<WfJob>& j
         auto launch_extend = [&](int it) {
             lt.mark(KC_EXTEND, st, true);
             if (it == 0 && packets)
-                wf_camera<COUNT, ONE><<<occ.grid_packet, blk, 0, st>>>(A, path_begin, (int)slots);
+                wf_camera<COUNT, ONE, KEEP><<<occ.grid_packet, blk, 0, st>>>(A, path_begin, (int)slots);
             else
-                wf_extend<COUNT, ONE><<<occ.grid_extend, blk, smem, st>>>(A, it);
+                wf_extend<COUNT, ONE, KEEP><<<occ.grid_extend, blk, smem, st>>>(A, it);
             lt.mark(KC_EXTEND, st, false);
         };
         if (iters > 0) launch_extend(0);
@@ -1222,7 +1251,7 @@ static cudaError_t enqueue_frame(const WfScratch& W, const std::vector<WfJob>& j
             if (sort_next &&
                 (e = cudaMemsetAsync(A.hist_e, 0, (size_t)kSortBinsE * 4, st)) != cudaSuccess)
                 return e;
-            wf_shade<COUNT, ONE><<<occ.grid_shade, blk, 0, st>>>(A, it);
+            wf_shade<COUNT, ONE, KEEP><<<occ.grid_shade, blk, 0, st>>>(A, it);
             if (A.sort_key >= 2) {
                 wf_sort_scan<<<kSortChunks, kSortChunk, 0, st>>>(A.hist_s, A.chunk_off);
                 wf_sort_chunks<kSortChunks><<<1, kSortChunk, 0, st>>>(A.chunk_off);
@@ -1243,12 +1272,12 @@ static cudaError_t enqueue_frame(const WfScratch& W, const std::vector<WfJob>& j
             if (overlap) {
                 if ((e = cudaEventRecord(W.ev_shaded, st)) != cudaSuccess) return e;
                 if ((e = cudaStreamWaitEvent(W.side, W.ev_shaded, 0)) != cudaSuccess) return e;
-                wf_shadow<COUNT, ONE><<<occ.grid_shadow, blk, smem, W.side>>>(A, it);
+                wf_shadow<COUNT, ONE, KEEP><<<occ.grid_shadow, blk, smem, W.side>>>(A, it);
                 if ((e = cudaEventRecord(W.ev_shadow, W.side)) != cudaSuccess) return e;
                 if (it + 1 < iters) launch_extend(it + 1);
             } else {
                 lt.mark(KC_SHADOW, st, true);
-                wf_shadow<COUNT, ONE><<<occ.grid_shadow, blk, smem, st>>>(A, it);
+                wf_shadow<COUNT, ONE, KEEP><<<occ.grid_shadow, blk, smem, st>>>(A, it);
                 lt.mark(KC_SHADOW, st, false);
                 if (it + 1 < iters) launch_extend(it + 1);
             }
@@ -1256,11 +1285,15 @@ static cudaError_t enqueue_frame(const WfScratch& W, const std::vector<WfJob>& j
         }
         if (overlap && iters > 0 && (e = cudaStreamWaitEvent(st, W.ev_shadow, 0)) != cudaSuccess)
             return e;
+        n_launch += 1;
+        if (finish) {
+            if ((e = (*finish)(pix_begin, pixels)) != cudaSuccess) return e;
+            continue;
+        }
         const unsigned ablocks = accumulate_blocks(pixels, occ.grid_accumulate, blk);
         lt.mark(KC_ACCUMULATE, st, true);
         wf_accumulate<<<ablocks, blk, 0, st>>>(A, pix_begin, (int)pixels, path_begin);
         lt.mark(KC_ACCUMULATE, st, false);
-        n_launch += 1;
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if (launches) *launches = n_launch;
@@ -1342,12 +1375,7 @@ cudaError_t wavefront_render(WfScratch& W, const std::vector<SceneView>& views,
                              cudaMemcpyHostToDevice, st)) != cudaSuccess)
         return e;
     if ((e = cudaMemsetAsync(W.args.status, 0, 4, st)) != cudaSuccess) return e;
-    if (!W.side) {
-        if ((e = cudaStreamCreateWithFlags(&W.side, cudaStreamNonBlocking)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&W.ev_shaded, cudaEventDisableTiming)) != cudaSuccess ||
-            (e = cudaEventCreateWithFlags(&W.ev_shadow, cudaEventDisableTiming)) != cudaSuccess)
-            return e;
-    }
+    if ((e = ensure_streams(W)) != cudaSuccess) return e;
     // A graph is reused while the frame's shape is unchanged.
     unsigned long long key = 1469598103934665603ull;
     auto mix = [&](unsigned long long v) { key = (key ^ v) * 1099511628211ull; };
@@ -1454,6 +1482,98 @@ cudaError_t wavefront_render(WfScratch& W, const std::vector<SceneView>& views,
     return cudaSuccess;
 }
 
+static cudaError_t ensure_streams(WfScratch& W) {
+    cudaError_t e;
+    if (W.side) return cudaSuccess;
+    if ((e = cudaStreamCreateWithFlags(&W.side, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&W.ev_shaded, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&W.ev_shadow, cudaEventDisableTiming)) != cudaSuccess)
+        return e;
+    return cudaSuccess;
+}
+
+cudaError_t launch_adjoint_found(const SceneView& S, const RenderCfg& c, const AdjointOut& o,
+                                 const float4* hit, const unsigned* vis, size_t stride,
+                                 long long pix_begin, long long pixels, cudaStream_t st);
+
+// The adjoint with its rays traced by the queued kernels: a chunk's paths run
+// forward once, every bounce's hits and shadow results kept (20 bytes per path
+// and bounce), and the replay that differentiates them traces nothing. The
+// kernel that traces as it replays keeps 5 of a warp's 32 lanes busy, as the
+// megakernel does. Per gradient of the box of 1,000 spheres, one kernel /
+// this: 17.3 / 11.6 ms at 4.2M paths, 4.64 / 3.43 at 1.05M, 3.67 / 2.27 at 590k,
+// 1.32 / 1.32 at 262k (100 spheres 0.61 / 0.79), 0.66 / 0.89 at 120k; so frames
+// of up to kAdjOneKernel paths keep the one kernel, and so do counting calls
+// and scenes whose vertices have more records than a word has bits. Sets
+// *done where the pass was made. The replay's arithmetic and the order of its
+// sums are the same.
+cudaError_t wavefront_adjoint(WfScratch& W, const SceneView& view,
+                              const std::vector<DevLight>& lights, const RenderCfg& cfg,
+                              const AdjointOut& o, cudaStream_t st, int* launches, bool* done) {
+    *done = false;
+    const long long paths = cfg.pixels() * cfg.spp;
+    const int maxS = max_shadow_records(view, lights, cfg.soft);
+    if (cfg.count || cfg.depth < 1 || maxS > 32 || paths <= kAdjOneKernel || cfg.spp > kAdjChunk)
+        return cudaSuccess;
+    const long long ppc = std::min<long long>(kAdjChunk / cfg.spp, cfg.pixels());
+    const int Q = (int)(ppc * cfg.spp);
+    const size_t per = al((size_t)Q * 16), per_vis = al((size_t)Q * 4);
+    const size_t need = (per + per_vis) * (size_t)cfg.depth;
+    cudaError_t e = ensure_scratch(W, Q, maxS, cfg.depth, 1, 1);
+    if (e == cudaSuccess && W.kept_bytes < need) {
+        if (W.kept) cudaFree(W.kept);
+        W.kept_bytes = 0;
+        e = cudaMalloc(&W.kept, need);
+        if (e == cudaSuccess) W.kept_bytes = need;
+        else W.kept = nullptr;
+    }
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();       // the kernel that needs no scratch does it
+        return cudaSuccess;
+    }
+    if (e != cudaSuccess || (e = ensure_streams(W)) != cudaSuccess) return e;
+    std::vector<WfJob> jobs(1);
+    WfJob& J = jobs[0];
+    J.P = PathParams{cfg.W, cfg.H, cfg.n, cfg.spp, cfg.depth, cfg.mode, cfg.rng, cfg.glass,
+                     cfg.soft, cfg.bias, cfg.salt, cfg.sample_offset, 0, 0, 0, 0, 0, 0};
+    J.view = 0;
+    J.path_off = J.pix_off = 0;
+    J.G = lanes_for(cfg.spp);
+    J.out = J.m2 = nullptr;
+    // this pass's arguments beside the renders' (whose graph keeps its own)
+    const WfArgs saved = W.args;
+    const int saved_block = W.block;
+    WfArgs& A = W.args;
+    A.hit = static_cast<float4*>(W.kept);
+    A.vis = reinterpret_cast<unsigned*>(static_cast<unsigned char*>(W.kept) + per * cfg.depth);
+    A.keep = per / 16;
+    A.n_jobs = 1;
+    A.counters = o.counters;
+    A.sort_key = cfg.sort_key ? cfg.sort_key : 3;
+    A.packets = 1;
+    A.refill_below = cfg.refill > 0 ? cfg.refill : 16;
+    A.maxS = maxS;
+    A.shadow_list = 1;
+    A.view0 = view;
+    A.job0 = J;
+    W.block = cfg.block > 0 ? cfg.block : kWfBlock;
+    LaunchTimer lt;
+    const float4* hit = A.hit;
+    const unsigned* vis = A.vis;
+    const size_t stride = A.keep;
+    const std::function<cudaError_t(long long, long long)> finish = [&](long long pix,
+                                                                         long long n) {
+        return launch_adjoint_found(view, cfg, o, hit, vis, stride, pix, n, st);
+    };
+    e = cudaMemsetAsync(A.status, 0, 4, st);
+    if (e == cudaSuccess)
+        e = enqueue_frame<false, true, true>(W, jobs, cfg.depth, Q, st, launches, lt, &finish);
+    W.args = saved;
+    W.block = saved_block;
+    *done = e == cudaSuccess;
+    return e;
+}
+
 void wavefront_release(WfScratch& W) {
     if (W.graph) cudaGraphExecDestroy(W.graph);
     W.graph = nullptr;
@@ -1461,6 +1581,9 @@ void wavefront_release(WfScratch& W) {
     W.mem = nullptr;
     W.bytes = 0;
     W.Q = 0;
+    if (W.kept) cudaFree(W.kept);
+    W.kept = nullptr;
+    W.kept_bytes = 0;
 }
 
 WfScratch* wavefront_new() { return new WfScratch(); }
@@ -1624,9 +1747,9 @@ cudaError_t wavefront_render_static(int device, const SceneView& view, const Dev
         wf_generate<false, true><<<(unsigned)((slots + kWfBlock - 1) / kWfBlock), kWfBlock, 0, st>>>(
             A, path0, (int)slots);
         for (int it = 0; it < c.depth; ++it) {
-            wf_extend<false, true><<<occ.grid_extend, kWfBlock, smem, st>>>(A, it);
-            wf_shade<false, true><<<occ.grid_shade, kWfBlock, 0, st>>>(A, it);
-            wf_shadow<false, true><<<occ.grid_shadow, kWfBlock, smem, st>>>(A, it);
+            wf_extend<false, true, false><<<occ.grid_extend, kWfBlock, smem, st>>>(A, it);
+            wf_shade<false, true, false><<<occ.grid_shade, kWfBlock, 0, st>>>(A, it);
+            wf_shadow<false, true, false><<<occ.grid_shadow, kWfBlock, smem, st>>>(A, it);
         }
         wf_accumulate<<<accumulate_blocks(pixels, occ.grid_accumulate), kWfBlock, 0, st>>>(
             A, pix0, (int)pixels, path0);

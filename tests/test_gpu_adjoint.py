@@ -170,3 +170,37 @@ def test_inverse_rendering_box_200_adam_steps(gpu):
           f"mean |albedo error| of {nv} visible spheres {err0:.4f} -> {err:.4f}")
     assert loss1 < 0.25 * loss0
     assert err < 0.5 * err0
+
+
+@pytest.mark.parametrize("name,size,depth,pathtrace", [
+    ("prims_mix", (171, 171, 3), 6, True), ("prims_mix", (171, 171, 3), 4, False),
+    ("three_spheres", (257, 256, 2), 16, True), ("adjoint_small", (256, 257, 2), 5, True),
+    ("cloud2k", (345, 331, 7), 2, True), ("cornell_box", (300, 225, 8), 1, True)])
+def test_adjoint_from_the_queued_kernels_is_the_traced_one(gpu, name, size, depth, pathtrace):
+    """Frames of more than 2^18 paths take hits and visibility from the
+    wavefront kernels (the last two in two chunks, of 49 and 64 samples a
+    pixel); counting calls trace in one kernel. The same image, and the same
+    gradients up to the order of the FP64 atomics."""
+    from conftest import load_golden
+    import dataclasses
+    w, h, n = size
+    scene, fx = load_golden(name)
+    if name == "adjoint_small":
+        w0, _, _ = W.adjoint_box(60, w, h, n, depth, seed=9)      # with its quad light
+        scene = w0.scene
+    st = RenderSettings(width=w, height=h, samples=n, max_depth=depth, pathtrace=pathtrace,
+                        pathtrace_bounces=depth, seed=11)
+    assert w * h * n * n > 1 << 18
+    sid = gpu.upload(scene)
+    dl = np.random.default_rng(2).normal(size=(h, w, 3)).astype(np.float32)
+    nm, nl = scene.n_materials, len(scene.lights)
+    a = gpu.adjoint(sid, st, dl, nm, nl, want_image=True)
+    b = gpu.adjoint(sid, dataclasses.replace(st, count_rays=True), dl, nm, nl, want_image=True)
+    assert np.array_equal(a[3].view(np.uint32), b[3].view(np.uint32))
+    for x, y in zip(a[:3], b[:3]):
+        # sums of at most 2^23 terms in FP64 in another order
+        assert np.abs(x - y).max() <= 1e-9 * max(np.abs(y).max(), 1e-30)
+    # and the context's renders are what they were
+    img = gpu.render(sid, st)
+    assert np.array_equal(img, gpu.render(sid, dataclasses.replace(st, block_size=128)))
+    gpu.free(sid)
