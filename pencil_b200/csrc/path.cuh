@@ -215,6 +215,12 @@ struct NeeAccum {
     }
 };
 
+// Whether a shadow ray can change nothing: the term it decides is zero (a
+// light behind the surface, a black albedo), and adding zero leaves a sum as
+// it is. About half of a lit vertex's lights are behind it; counting renders
+// trace such rays all the same, as the reference does.
+__device__ __forceinline__ bool no_term(V3 c) { return c.x == 0.0f && c.y == 0.0f && c.z == 0.0f; }
+
 // Shade one vertex of a single-ray path and choose its continuation.
 // `found`/`h` is the closest hit of ps.ray. Next-event shadow rays go to
 // E.shadow(L, ray, tmin, tmax, test, c, group_end) in order and the terms
@@ -373,8 +379,9 @@ struct Tracer {
         bool vis = false;
         V3 c = v3(0, 0, 0);
         if (me < t.n) {
-            vis = S.lights[t.light].is_emissive || !occluded(Ray{sorg, t.L}, P.bias, t.tmax);
-            if (vis) c = term(t);
+            c = term(t);
+            vis = S.lights[t.light].is_emissive || (!COUNT && no_term(c)) ||
+                  !occluded(Ray{sorg, t.L}, P.bias, t.tmax);
         }
         const unsigned v = __ballot_sync(mask, vis) >> base;
         for (int q = 0; q < t.n; ++q) {
@@ -422,7 +429,6 @@ struct Tracer {
                 light_dir(l, h.p, rng, L, dist);
                 if (!shade) continue;
                 Ray sr{h.p + h.n * P.bias, L};
-                if (!l.is_emissive && occluded(sr, P.bias, dist - P.bias)) continue;
                 float ndotl = clampf(dot(h.n, L), 0.0f, 1.0f);
                 V3 c = albedo * ld3(l.intensity) * ndotl;
                 if (m.specular > 0.0f && ndotl > 0.0f) {
@@ -432,6 +438,8 @@ struct Tracer {
                     float spec = powf(ndoth, m.shininess);
                     c = c + ld3(m.specular_color) * ld3(l.intensity) * (spec * m.specular);
                 }
+                if (!COUNT && no_term(c)) continue;
+                if (!l.is_emissive && occluded(sr, P.bias, dist - P.bias)) continue;
                 contrib = contrib + c;
             }
             local = local + contrib / (float)ns;
@@ -664,9 +672,11 @@ struct Tracer {
             float dist;
             light_dir(l, h.p, rng, L, dist);
             Ray sr{h.p + h.n * P.bias, L};
-            if (!l.is_emissive && occluded(sr, P.bias, dist - P.bias)) continue;
             float ndotl = clampf(dot(h.n, L), 0.0f, 1.0f);
-            rad = rad + light_term(l, P.mis != 0, T, albedo, L, dist, ndotl);
+            const V3 c = light_term(l, P.mis != 0, T, albedo, L, dist, ndotl);
+            if (!COUNT && no_term(c)) continue;
+            if (!l.is_emissive && occluded(sr, P.bias, dist - P.bias)) continue;
+            rad = rad + c;
         }
         if (quad_nee) {
             for (int li = 0; li < S.n_lights; ++li) {
@@ -722,7 +732,7 @@ struct Tracer {
         __device__ __forceinline__ void begin_whitted(V3 base) { acc.begin_whitted(base); }
         __device__ __forceinline__ void shadow(V3& L, const Ray& sr, float tmin, float tmax,
                                                bool test, V3 c, int group_end) {
-            bool vis = !test || !tr.occluded(sr, tmin, tmax);
+            bool vis = !test || (!COUNT && no_term(c)) || !tr.occluded(sr, tmin, tmax);
             acc.add(L, c, group_end, vis);
         }
         __device__ __forceinline__ void pending(V3 tl, V3 ww, float ss) { tail = tl; w = ww; s = ss; }

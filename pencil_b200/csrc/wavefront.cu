@@ -576,6 +576,9 @@ __global__ void __launch_bounds__(kWfMaxBlock) wf_camera(WfArgs A, long long pat
 
 // ---- shade --------------------------------------------------------------------
 // Emitter that stores a vertex's shadow records and pending terms per slot.
+// SKIP: records whose term is zero are not made (a Whitted vertex keeps them,
+// untested, for the ends of its lights' groups).
+template <bool SKIP>
 struct StoreNee {
     const WfArgs& A;
     int slot;
@@ -592,6 +595,10 @@ struct StoreNee {
     __device__ __forceinline__ void begin_whitted(V3 b) { kind = 2; base = b; }
     __device__ __forceinline__ void shadow(V3&, const Ray& r, float tmin, float tmax, bool test,
                                            V3 c, int group_end) {
+        if (SKIP && no_term(c)) {
+            if (kind == 1) return;
+            test = false;
+        }
         if (n >= A.maxS) {
             atomicOr(A.status, 1);
             return;
@@ -626,6 +633,7 @@ wf_shade(WfArgs A, int it) {
     unsigned int* cursor = A.work + it * 3 + 1;
     int* qout = A.q[(it + 1) & 1];
     int* cout = A.counts + (it + 1) * kOctants;
+    const bool listed = A.sort_key >= 2 || A.shadow_list;   // else shadow looks at every slot
     const int lane = threadIdx.x & 31;
     while (true) {
         int base = fetch32(cursor);
@@ -657,10 +665,16 @@ wf_shade(WfArgs A, int it) {
             Hit h;
             bool found = leaf >= 0;
             if (found) make_hit(S, __float_as_int(hv.y), leaf, ps.ray, 1e-4f, hv.x, h);
-            StoreNee E(A, slot);
+            constexpr bool SKIP = !COUNT && !KEEP;
+            StoreNee<SKIP> E(A, slot);
             alive = shade_vertex(S, J.P, ps, found, h, E);
-            E.store();
+            if (SKIP && E.kind == 1 && E.n == 0) {
+                // no shadow ray: the pending term is due at once
+                ps.L = ps.L + E.tail;
+                E.kind = 0;
+            }
             shadow_work = E.kind != 0;
+            if (shadow_work || !listed) E.store();
             if (A.sort_key >= 2 && shadow_work) key = sort_key_of(S, E.o0, E.d0);
             if (COUNT && alive && (ps.flags & kFlagWhitted)) rc.ref++;
             A.L[slot] = make_float4(ps.L.x, ps.L.y, ps.L.z, 0.0f);
@@ -677,7 +691,7 @@ wf_shade(WfArgs A, int it) {
         }
         // the list of slots with shadow work; sort key 2: with their keys,
         // ordered by wf_sort_scatter
-        if (A.sort_key >= 2 || A.shadow_list)
+        if (listed)
             warp_append(shadow_work, slot, A.tcnt + 2 * it + 1, A.tmp_s, lane,
                         A.sort_key >= 2 ? A.key_s : nullptr, key);
         if (A.sort_key >= 2) {

@@ -111,3 +111,27 @@ def test_both_sides_of_the_one_kernel_line(gpu, side):
     b = gpu.render(sid, dataclasses.replace(st, block_size=128))
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     gpu.free(sid)
+
+
+@pytest.mark.parametrize("name", ["three_spheres", "prims_mix", "cloud2k", "cornell_box"])
+@pytest.mark.parametrize("pathtrace", [False, True])
+def test_shadow_rays_that_decide_nothing(gpu, name, pathtrace):
+    """Lights behind a surface, black albedos and black lights make no shadow
+    ray, except in counting renders: the same image from both, on the queues,
+    in one kernel and in the reference-exact mode."""
+    scene, _ = load_golden(name)
+    scene.add_light(Light.point((0.3, 2.5, -3.0), (0.0, 0.0, 0.0), 0.4))
+    scene.add_light(Light.directional((0.0, -1.0, 0.0), (0.4, 0.0, 0.2)))
+    m = scene.material_array().copy()
+    m["albedo"][0] = (0.0, 0.0, 0.0)
+    scene.set_material_array(m)
+    sid = gpu.upload(scene)
+    st = RenderSettings(width=83, height=61, samples=2, max_depth=5, pathtrace=pathtrace,
+                        pathtrace_bounces=5, seed=5)
+    exact = dict(engine=A.ENGINE_MEGAKERNEL, rng=A.RNG_PIXEL_SEQUENTIAL,
+                 glass=A.GLASS_BOTH_BRANCHES)
+    for kw in (dict(block_size=64), dict(sort_key=3), dict(), dict(mis=True), exact):
+        s = dataclasses.replace(st, **kw)
+        a, b = gpu.render(sid, s), gpu.render(sid, dataclasses.replace(s, count_rays=True))
+        assert np.array_equal(a, b), kw
+    gpu.free(sid)
