@@ -51,9 +51,9 @@ int adjoint_max_lights();
 cudaError_t launch_tonemap(const float* d_hdr, long long n_pixels, int mode, float exposure,
                            uint8_t* d_out, const void* d_table, cudaStream_t st);
 const void* tone_table_host(size_t* bytes);
-cudaError_t device_sah(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out, int& depth,
+cudaError_t device_sah(const pgpu_scene& s, int n_unified, pgpu_bvh_node* d_out, int* depth,
                        cudaStream_t st, cudaMemPool_t pool, bool quality);
-cudaError_t device_lbvh(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out, int& depth,
+cudaError_t device_lbvh(const pgpu_scene& s, int n_unified, pgpu_bvh_node* d_out, int* depth,
                         cudaStream_t st, cudaMemPool_t pool);
 
 constexpr int kMaxDepth = 64;          // traversal stack bound (kMaxStack)
@@ -139,6 +139,7 @@ struct pgpu_ctx {
     void* d_query = nullptr;
     size_t query_cap = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_tree = nullptr;    // an upload's traversal tree is on the host
     WfScratch* wf = nullptr;
     int* h_status = nullptr;          // pinned
     unsigned char* h_stage = nullptr; // pinned staging of scene uploads
@@ -164,7 +165,6 @@ struct pgpu_ctx {
     bool in_flight = false;
     // tree of the wide traversals of later uploads (pgpu_set_traversal_tree)
     int traversal = PGPU_TRAVERSAL_UPLOADED;
-    std::vector<pgpu_bvh_node> ws_trav;
     std::vector<int> ws_leaf_of_prim;
 };
 
@@ -228,7 +228,7 @@ int drain(pgpu_ctx* c) {
 // f(begin, end) over [0, n) on the host worker threads (one when n is small).
 template <class F>
 void parallel_for(int n, F f) {
-    constexpr int kGrain = 16384;
+    constexpr int kGrain = 8192;
     const int T = std::min(host_threads(), (n + kGrain - 1) / kGrain);
     if (T <= 1) { f(0, n); return; }
     const int chunk = (n + T - 1) / T;
@@ -296,6 +296,34 @@ int ensure(pgpu_ctx* c, T*& ptr, size_t& cap, size_t need) {
     }
     cap = std::max<size_t>(need, 256);
     return PGPU_OK;
+}
+
+// Pinned host memory of at least `need` bytes (contents lost when it grows).
+int ensure_pinned(pgpu_ctx* c, unsigned char*& p, size_t& cap, size_t need) {
+    if (cap >= need) return PGPU_OK;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+    if (cudaMallocHost(reinterpret_cast<void**>(&p), need) != cudaSuccess) {
+        (void)cudaGetLastError();
+        p = nullptr;
+        return fail(c, PGPU_ERR_OUT_OF_MEMORY, "pinned staging of %zu bytes", need);
+    }
+    cap = need;
+    return PGPU_OK;
+}
+
+// Touches every page of a result buffer that will be overwritten whole, on the
+// host threads, while the device is still making the result: the first write
+// to a fresh buffer's page faults, and the driver's copy into pageable memory
+// would take those faults one after the other (a table of 5.2 MB: 1.4 ms).
+void touch_pages(void* p, size_t bytes) {
+    constexpr size_t kPage = 4096, kPart = 64 * kPage;
+    if (bytes < 4 * kPart) return;
+    host_run((int)(bytes / kPart), [&](int t) {
+        volatile char* q = static_cast<volatile char*>(p) + t * kPart;
+        for (size_t b = 0; b < kPart; b += kPage) q[b] = 0;
+    });
 }
 
 DeviceScene* find_scene(pgpu_ctx* c, int id) {
@@ -405,6 +433,7 @@ int32_t pgpu_create(int32_t device, pgpu_ctx** out) {
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_tree, cudaEventDisableTiming) != cudaSuccess ||
         cudaMalloc(reinterpret_cast<void**>(&c->d_cnt), CNT_N * sizeof(unsigned long long)) !=
             cudaSuccess ||
         cudaMallocHost(reinterpret_cast<void**>(&c->h_status), 16) != cudaSuccess) {
@@ -440,6 +469,7 @@ void pgpu_destroy(pgpu_ctx* c) {
     if (c->h_stage) cudaFreeHost(c->h_stage);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
+    if (c->ev_tree) cudaEventDestroy(c->ev_tree);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
 }
@@ -499,33 +529,61 @@ int32_t pgpu_build_bvh(const pgpu_scene* s, pgpu_bvh_node* out_nodes, int32_t* o
 
 }  // extern "C"
 
-// The traversal tree of an upload (PGPU_TRAVERSAL_LBVH / _SAH): built on the
-// device over the scene's primitives, checked to be a DFS table over every
+// Enqueues a device build of mode `mode` (PGPU_TRAVERSAL_LBVH, _SAH; `pencil`:
+// Pencil's SAH tree) into a table from the context's pool (*d_table, to be
+// freed on the stream) and its copy to `host` (pinned; null: none).
+static cudaError_t start_tree(pgpu_ctx* c, const pgpu_scene& s, int nU, int mode, bool pencil,
+                              pgpu_bvh_node** d_table, pgpu_bvh_node* host) {
+    const size_t bytes = (2 * (size_t)nU - 1) * sizeof(pgpu_bvh_node);
+    *d_table = nullptr;
+    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(d_table), bytes, c->pool,
+                                            c->stream);
+    if (e != cudaSuccess) { *d_table = nullptr; return e; }
+    int* depth = c->h_status + 2;
+    e = mode == PGPU_TRAVERSAL_SAH
+            ? device_sah(s, nU, *d_table, depth, c->stream, c->pool, !pencil)
+            : device_lbvh(s, nU, *d_table, depth, c->stream, c->pool);
+    if (e == cudaSuccess && host)
+        e = cudaMemcpyAsync(host, *d_table, bytes, cudaMemcpyDeviceToHost, c->stream);
+    return e;
+}
+
+// The traversal tree of an upload (PGPU_TRAVERSAL_LBVH / _SAH), in T: built on
+// the device over the scene's primitives, checked to be a DFS table over every
 // primitive once, then given the uploaded tree's leaf boxes -- the builder's
 // boxes are the same primitive boxes; where one differs in a bit, the
 // uploaded one is taken and the interior boxes are refit as unions, so
 // every box still contains its subtree's. leaf_of[p] receives the uploaded
 // tree's leaf of primitive p.
-static int traversal_tree(pgpu_ctx* c, const pgpu_scene& s, const pgpu_bvh_node* nodes,
-                          int n_nodes, int nU, int mode, std::vector<int>& leaf_of,
-                          std::vector<pgpu_bvh_node>& T) {
+static int traversal_tree(pgpu_ctx* c, const pgpu_bvh_node* nodes, int n_nodes, int nU,
+                          std::vector<int>& leaf_of, pgpu_bvh_node* T) {
     leaf_of.assign(nU, -1);
+    // (both loops wait for scattered reads and writes: fetched some nodes ahead)
+    constexpr int kAhead = 24;
     parallel_for(n_nodes, [&](int b, int e) {
-        for (int k = b; k < e; ++k)
+        for (int k = b; k < e; ++k) {
+            if (k + kAhead < e && nodes[k + kAhead].left < 0)
+                __builtin_prefetch(&leaf_of[nodes[k + kAhead].right], 1);
             if (nodes[k].left < 0) leaf_of[nodes[k].right] = k;
+        }
     });
-    T.resize(n_nodes);
-    int depth = 0;
-    const cudaError_t e = mode == PGPU_TRAVERSAL_SAH
-                              ? device_sah(s, nU, T.data(), depth, c->stream, c->pool, true)
-                              : device_lbvh(s, nU, T.data(), depth, c->stream, c->pool);
-    if (e != cudaSuccess) return cuda_fail(c, e, "traversal tree build");
     std::vector<char>& seen = c->ws_seen;
     seen.assign(nU, 0);
     std::atomic<int> bad{0}, differ{0};
     parallel_for(n_nodes, [&](int b, int e2) {
+        // the uploaded leaf of node k, -1 where it names none
+        auto leaf = [&](int k) {
+            return k < e2 && T[k].left < 0 && T[k].right >= 0 && T[k].right < nU
+                       ? leaf_of[T[k].right] : -1;
+        };
         for (int k = b; k < e2; ++k) {
-            const pgpu_bvh_node& t = T[k];
+            if (k + 2 * kAhead < e2 && T[k + 2 * kAhead].left < 0 &&
+                (unsigned)T[k + 2 * kAhead].right < (unsigned)nU) {
+                __builtin_prefetch(&leaf_of[T[k + 2 * kAhead].right]);
+                __builtin_prefetch(&seen[T[k + 2 * kAhead].right], 1);
+            }
+            if (const int f = leaf(k + kAhead); f >= 0) __builtin_prefetch(&nodes[f]);
+            pgpu_bvh_node& t = T[k];
             if (t.left >= 0) {
                 if (t.left != k + 1 || t.right <= k + 1 || t.right >= n_nodes) bad = 1;
                 continue;
@@ -533,20 +591,20 @@ static int traversal_tree(pgpu_ctx* c, const pgpu_scene& s, const pgpu_bvh_node*
             if (t.right < 0 || t.right >= nU || leaf_of[t.right] < 0) { bad = 1; continue; }
             // one leaf per primitive: a primitive's flag is set by one leaf only
             if (__atomic_exchange_n(&seen[t.right], (char)1, __ATOMIC_RELAXED)) { bad = 1; continue; }
+            // the uploaded leaf's box bit for bit; boxes that differ in the sign
+            // of a zero alone bound the same points
             const pgpu_bvh_node& u = nodes[leaf_of[t.right]];
-            if (std::memcmp(t.bmin, u.bmin, 12) || std::memcmp(t.bmax, u.bmax, 12)) differ = 1;
+            for (int a = 0; a < 3; ++a)
+                if (t.bmin[a] != u.bmin[a] || t.bmax[a] != u.bmax[a]) differ = 1;
+            std::memcpy(t.bmin, u.bmin, 12);
+            std::memcpy(t.bmax, u.bmax, 12);
         }
     });
     if (bad) return fail(c, PGPU_ERR_BVH_INVALID, "device traversal tree is not a DFS table");
     if (differ) {
         for (int k = n_nodes - 1; k >= 0; --k) {
             pgpu_bvh_node& t = T[k];
-            if (t.left < 0) {
-                const pgpu_bvh_node& u = nodes[leaf_of[t.right]];
-                std::memcpy(t.bmin, u.bmin, 12);
-                std::memcpy(t.bmax, u.bmax, 12);
-                continue;
-            }
+            if (t.left < 0) continue;
             const pgpu_bvh_node &l = T[t.left], &r = T[t.right];
             for (int a = 0; a < 3; ++a) {
                 t.bmin[a] = std::fmin(l.bmin[a], r.bmin[a]);
@@ -589,11 +647,19 @@ static int32_t build_bvh_device(pgpu_ctx* c, const pgpu_scene* s, pgpu_bvh_node*
     }
     PGPU_CUDA(c, cudaSetDevice(c->device));
     PGPU_CUDA(c, ensure_pool(c));
-    int depth = 0;
-    cudaError_t e = sah ? device_sah(*s, n, out_nodes, depth, c->stream, c->pool, false)
-                        : device_lbvh(*s, n, out_nodes, depth, c->stream, c->pool);
+    pgpu_bvh_node* d_table = nullptr;
+    cudaError_t e = start_tree(c, *s, n, sah ? PGPU_TRAVERSAL_SAH : PGPU_TRAVERSAL_LBVH, true,
+                               &d_table, nullptr);
+    const size_t bytes = (2 * (size_t)n - 1) * sizeof(pgpu_bvh_node);
+    if (e == cudaSuccess) {
+        touch_pages(out_nodes, bytes);
+        e = cudaMemcpyAsync(out_nodes, d_table, bytes, cudaMemcpyDeviceToHost, c->stream);
+    }
+    if (d_table) cudaFreeAsync(d_table, c->stream);
+    const cudaError_t se = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = se;
     if (e != cudaSuccess) return cuda_fail(c, e, "device BVH build");
-    if (out_depth) *out_depth = depth;
+    if (out_depth) *out_depth = c->h_status[2];
     return PGPU_OK;
 }
 
@@ -713,12 +779,6 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
         nodes = built.data();
         n_nodes = (int)built.size();
     }
-    int rc = check_tree(c, nodes, n_nodes, nU, depth);
-    if (rc) return rc;
-
-    // DFS order numbering of interior nodes and leaf slots (check_tree)
-    const std::vector<int>& idx = c->ws_idx;
-    const int n_leaf = nU, n_int = nU > 0 ? nU - 1 : 0;
     // triangles keep their first vertex and both edges (v1 - v0, v2 - v0, the
     // reference's first two operations, rounded alike here) in their leaf
     // slot (geo_a, geo_b, geo_c): a triangle test then loads them directly,
@@ -727,17 +787,12 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     const bool has_tri = s->n_mesh_triangles > 0 || first_bad(s->n_prims, [&](int k) {
         return s->prims[k].type == PGPU_PRIM_TRIANGLE;
     }) >= 0;
+    const int n_leaf = nU, n_int = nU > 0 ? nU - 1 : 0;
 
-    auto ref_of = [&](int k) -> int {
-        if (nodes[k].left >= 0) return idx[k];
-        int prim = nodes[k].right;
-        int type = prim < s->n_prims ? s->prims[prim].type : PGPU_PRIM_TRIANGLE;
-        return ~((type << kLeafTypeShift) | idx[k]);
-    };
-
-    // Staging: the main arena's bytes, then room for one wide node per
-    // binary interior node (the most the collapse can make). The main part
-    // is copied to the device while the wide nodes are being built.
+    // Staging: the main arena's bytes, room for one wide node per binary
+    // interior node (the most the collapse can make), and a device-built
+    // traversal tree's table. The main part is copied to the device while the
+    // wide nodes are being built.
     size_t off_nodes = 0;
     size_t off_ga = align256(off_nodes + (size_t)n_int * 64);
     size_t off_gb = align256(off_ga + (size_t)n_leaf * 16);
@@ -748,17 +803,46 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     size_t off_mt = align256(off_lp + (size_t)n_leaf * 4);
     size_t off_lt = align256(off_mt + (size_t)s->n_materials * sizeof(DevMaterial));
     size_t total = align256(off_lt + lights.size() * sizeof(DevLight));
-    const size_t wide_cap = (size_t)n_int * kWideNodeFloat4 * 16;
-    if (c->stage_cap < total + wide_cap) {
-        if (c->h_stage) cudaFreeHost(c->h_stage);
-        c->h_stage = nullptr;
-        c->stage_cap = 0;
-        if (cudaMallocHost(reinterpret_cast<void**>(&c->h_stage), total + wide_cap) != cudaSuccess) {
-            c->h_stage = nullptr;
-            return fail(c, PGPU_ERR_OUT_OF_MEMORY, "pinned staging of %zu bytes", total + wide_cap);
+    const size_t wide_cap = align256((size_t)n_int * kWideNodeFloat4 * 16);
+    const bool own_tree = c->traversal != PGPU_TRAVERSAL_UPLOADED && nU >= 2;
+    const size_t tree_cap = own_tree ? (2 * (size_t)nU - 1) * sizeof(pgpu_bvh_node) : 0;
+    int rc = ensure_pinned(c, c->h_stage, c->stage_cap, total + wide_cap + tree_cap);
+    if (rc) return rc;
+    // A traversal tree of its own needs only the primitives: the device builds
+    // it while the host checks and converts the uploaded one (82k triangles:
+    // 4.3 -> 3.9 ms for the upload). Whatever fails below waits for it.
+    struct TreeGuard {
+        pgpu_ctx* c;
+        pgpu_bvh_node* d = nullptr;
+        bool pending = false;
+        ~TreeGuard() {
+            if (d) cudaFreeAsync(d, c->stream);
+            if (pending) cudaStreamSynchronize(c->stream);
         }
-        c->stage_cap = total + wide_cap;
+    } tree{c};
+    pgpu_bvh_node* h_tree = reinterpret_cast<pgpu_bvh_node*>(c->h_stage + total + wide_cap);
+    if (own_tree) {
+        PGPU_CUDA(c, cudaSetDevice(c->device));
+        PGPU_CUDA(c, ensure_pool(c));
+        tree.pending = true;
+        const cudaError_t te = start_tree(c, *s, nU, c->traversal, false, &tree.d, h_tree);
+        if (te != cudaSuccess) return cuda_fail(c, te, "traversal tree build");
+        PGPU_CUDA(c, cudaEventRecord(c->ev_tree, c->stream));
     }
+
+    rc = check_tree(c, nodes, n_nodes, nU, depth);
+    if (rc) return rc;
+
+    // DFS order numbering of interior nodes and leaf slots (check_tree)
+    const std::vector<int>& idx = c->ws_idx;
+
+    auto ref_of = [&](int k) -> int {
+        if (nodes[k].left >= 0) return idx[k];
+        int prim = nodes[k].right;
+        int type = prim < s->n_prims ? s->prims[prim].type : PGPU_PRIM_TRIANGLE;
+        return ~((type << kLeafTypeShift) | idx[k]);
+    };
+
     unsigned char* host = c->h_stage;
     // every byte is written below except the alignment gaps; those are
     // zeroed so that uploads are deterministic
@@ -892,11 +976,13 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     // the uploaded tree's leaf boxes and slots.
     const pgpu_bvh_node* tnodes = nodes;
     std::vector<int>& leaf_of = c->ws_leaf_of_prim;    // primitive -> its leaf in `nodes`
-    const bool own_tree = c->traversal != PGPU_TRAVERSAL_UPLOADED && nU >= 2;
     if (own_tree) {
-        rc = traversal_tree(c, *s, nodes, n_nodes, nU, c->traversal, leaf_of, c->ws_trav);
+        // the stream has the tree's copy before the main arena's
+        e = cudaEventSynchronize(c->ev_tree);
+        if (e == cudaSuccess) rc = traversal_tree(c, nodes, n_nodes, nU, leaf_of, h_tree);
+        else rc = cuda_fail(c, e, "traversal tree build");
         if (rc) { release(); return rc; }
-        tnodes = c->ws_trav.data();
+        tnodes = h_tree;
     }
     // 4-wide nodes, built while the main part is in flight
     std::vector<int>& leaf_ref = c->ws_leaf_ref;

@@ -1043,9 +1043,11 @@ __global__ void sah_root(const int* bounds, int n, int local_max, SahTask* tasks
 
 }  // namespace
 
-// Builds the table on the current device; n_unified >= 2. Device memory for
-// the build is allocated here and freed before returning.
-cudaError_t device_lbvh(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out, int& depth,
+// Enqueues the build of the table on the current device; n_unified >= 2. The
+// table (device memory, 2 n_unified - 1 rows) and its depth (pinned host
+// memory) are valid once `st` has finished, and so the inputs are read.
+// Device memory for the build is allocated here and returned in stream order.
+cudaError_t device_lbvh(const pgpu_scene& s, int n_unified, pgpu_bvh_node* d_out, int* depth,
                         cudaStream_t st, cudaMemPool_t pool) {
     const int n = n_unified;
     const size_t np = (size_t)s.n_prims, nv = (size_t)s.n_mesh_vertices,
@@ -1056,7 +1058,7 @@ cudaError_t device_lbvh(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out, 
     size_t bytes = al(np * sizeof(pgpu_prim)) + al(nv * 12) + al(nt * 12) +
                    al((size_t)n * sizeof(DBox)) + al(6 * 4) + 2 * al((size_t)n * 8) +
                    3 * al(total * 4) + al(total * sizeof(DBox)) + 3 * al(total * 4) +
-                   al((size_t)n * 4) + al(4) + al(total * sizeof(pgpu_bvh_node));
+                   al((size_t)n * 4) + al(4);
     size_t sort_bytes = 0;
     cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, (unsigned long long*)nullptr,
                                    (unsigned long long*)nullptr, n, 0, 64, st);
@@ -1082,7 +1084,6 @@ cudaError_t device_lbvh(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out, 
     auto* d_level = reinterpret_cast<int*>(take(total * 4));
     auto* d_arrive = reinterpret_cast<int*>(take((size_t)n * 4));
     auto* d_maxlvl = reinterpret_cast<int*>(take(4));
-    auto* d_out = reinterpret_cast<pgpu_bvh_node*>(take(total * sizeof(pgpu_bvh_node)));
     void* d_sort_tmp = take(sort_bytes);
 
     if (np) e = cudaMemcpyAsync(d_prims, s.prims, np * sizeof(pgpu_prim), cudaMemcpyHostToDevice, st);
@@ -1111,19 +1112,14 @@ cudaError_t device_lbvh(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out, 
                                        d_pre, d_level, d_maxlvl);
     lb_write<<<grid(total), B, 0, st>>>(d_sorted, n, d_left, d_right, d_nbox, d_pre, d_out);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(out, d_out, total * sizeof(pgpu_bvh_node),
-                             cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-        return e;
-    if ((e = cudaMemcpyAsync(&depth, d_maxlvl, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-        return e;
-    return cudaStreamSynchronize(st);
+    return cudaMemcpyAsync(depth, d_maxlvl, 4, cudaMemcpyDeviceToHost, st);
 }
 
-// Pencil's binned SAH tree, built on the current device; n_unified >= 2.
-// Device memory for the build is allocated here and freed before returning.
+// Pencil's binned SAH tree, built on the current device; n_unified >= 2. Waits
+// for its levels, but like device_lbvh not for the table's copy.
 template <bool Q>
-static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out,
-                                   int& depth, cudaStream_t st, cudaMemPool_t pool) {
+static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_node* d_out,
+                                   int* depth, cudaStream_t st, cudaMemPool_t pool) {
     constexpr int NB = kBinsPerTask<Q>;
     const int n = n_unified;
     const size_t np = (size_t)s.n_prims, nv = (size_t)s.n_mesh_vertices,
@@ -1150,8 +1146,7 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
                    al((size_t)t_max * sizeof(SahChoice)) + 2 * al((size_t)t_max * 4) +
                    2 * al((size_t)item_max * 4) + 3 * al((size_t)t_max * 4) +
                    2 * al((size_t)n * 4) + 2 * al((size_t)n * 4) +
-                   al((size_t)l_max * sizeof(SahTask)) +
-                   al(total * sizeof(pgpu_bvh_node)) + al(scan_bytes) + al(seg_bytes) + al(4 * 4);
+                   al((size_t)l_max * sizeof(SahTask)) + al(scan_bytes) + al(seg_bytes) + al(4 * 4);
     DevBuf mem;
     cudaError_t e = mem.alloc(bytes, pool, st);
     if (e != cudaSuccess) return e;
@@ -1181,7 +1176,6 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
     auto* d_keys2 = reinterpret_cast<float*>(take((size_t)n * 4));
     auto* d_vals = reinterpret_cast<int*>(take((size_t)n * 4));
     auto* d_vals2 = reinterpret_cast<int*>(take((size_t)n * 4));
-    auto* d_out = reinterpret_cast<pgpu_bvh_node*>(take(total * sizeof(pgpu_bvh_node)));
     void* d_scan_tmp = take(scan_bytes);
     void* d_seg_tmp = take(seg_bytes);
     int* d_misc = reinterpret_cast<int*>(take(4 * 4));   // small tasks, deepest level, local tasks
@@ -1299,18 +1293,13 @@ static cudaError_t device_sah_impl(const pgpu_scene& s, int n_unified, pgpu_bvh_
         sah_small<<<grid(host_ctr[0]), B, 0, st>>>(d_small, host_ctr[0], d_perm, d_boxes, d_out,
                                                   (int)total, d_misc + 1);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(out, d_out, total * sizeof(pgpu_bvh_node),
-                             cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-        return e;
-    if ((e = cudaMemcpyAsync(&depth, d_misc + 1, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess)
-        return e;
-    return cudaStreamSynchronize(st);
+    return cudaMemcpyAsync(depth, d_misc + 1, 4, cudaMemcpyDeviceToHost, st);
 }
 
-cudaError_t device_sah(const pgpu_scene& s, int n_unified, pgpu_bvh_node* out, int& depth,
+cudaError_t device_sah(const pgpu_scene& s, int n_unified, pgpu_bvh_node* d_out, int* depth,
                        cudaStream_t st, cudaMemPool_t pool, bool quality) {
-    return quality ? device_sah_impl<true>(s, n_unified, out, depth, st, pool)
-                   : device_sah_impl<false>(s, n_unified, out, depth, st, pool);
+    return quality ? device_sah_impl<true>(s, n_unified, d_out, depth, st, pool)
+                   : device_sah_impl<false>(s, n_unified, d_out, depth, st, pool);
 }
 
 }  // namespace pgpu

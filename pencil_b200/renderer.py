@@ -169,12 +169,14 @@ class GpuContext:
         fn = {"lbvh": "pgpu_build_bvh_device", "sah": "pgpu_build_bvh_device_sah"}[method]
         d, keep = scene.desc()
         n = scene.n_unified
-        nodes = np.zeros(max(2 * n - 1, 1), A.NODE_DTYPE)
+        nodes = np.empty(max(2 * n - 1, 0), A.NODE_DTYPE)
+        room = nodes if n else np.empty(1, A.NODE_DTYPE)
         cnt, depth = C.c_int32(0), C.c_int32(0)
-        self.check(getattr(self.lib, fn)(self.h, C.byref(d), A.ptr(nodes), C.byref(cnt),
+        self.check(getattr(self.lib, fn)(self.h, C.byref(d), A.ptr(room), C.byref(cnt),
                                          C.byref(depth)), fn)
         del keep
-        return nodes[: cnt.value].copy(), depth.value
+        assert cnt.value == len(nodes)        # one leaf per primitive
+        return nodes, depth.value
 
     def render_tile(self, sid: int, settings: RenderSettings, x: int, y: int, w: int,
                     h: int) -> np.ndarray:
