@@ -135,3 +135,27 @@ def test_shadow_rays_that_decide_nothing(gpu, name, pathtrace):
         a, b = gpu.render(sid, s), gpu.render(sid, dataclasses.replace(s, count_rays=True))
         assert np.array_equal(a, b), kw
     gpu.free(sid)
+
+
+def test_automatic_capacity_over_frames_of_many_shapes(gpu):
+    """One context, frames that grow the scratch by paths, then by records,
+    then shrink: every image as a fresh context renders it in small chunks."""
+    from pencil_b200.renderer import GpuContext
+    many, _ = load_golden("prims_mix")
+    for k in range(40):
+        many.add_light(Light.point((0.1 * k, 4.0, -3.0), (0.02, 0.02, 0.02), 0.0))
+    few, _ = load_golden("cloud2k")
+    a, b = gpu.upload(few), gpu.upload(many)
+    frames = [(a, few, 700, 500, 4), (b, many, 120, 90, 2), (a, few, 1200, 1100, 4),
+              (b, many, 300, 200, 3), (a, few, 97, 61, 1)]
+    ctx = GpuContext(0)
+    ca, cb = ctx.upload(few), ctx.upload(many)
+    for sid, scene, w, h, n in frames:
+        st = RenderSettings(width=w, height=h, samples=n, pathtrace=True, pathtrace_bounces=3,
+                            block_size=128)
+        img = gpu.render(sid, st)
+        ref = ctx.render(ca if sid == a else cb, dataclasses.replace(st, queue_capacity=1 << 18))
+        assert np.array_equal(img.view(np.uint32), ref.view(np.uint32)), (w, h, n)
+    ctx.close()
+    gpu.free(a)
+    gpu.free(b)
