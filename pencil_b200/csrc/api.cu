@@ -23,6 +23,8 @@ namespace pgpu {
 
 cudaError_t launch_megakernel(const SceneView& S, const RenderCfg& c, float* out, float* m2,
                               unsigned long long* counters, cudaStream_t st);
+cudaError_t launch_wide_relative(const float4* wide, int n_wide, const float* origin, float4* out,
+                                 cudaStream_t st);
 cudaError_t launch_query(const SceneView& S, bool camera, const float* in, int n, int* prim,
                          float* t, cudaStream_t st);
 
@@ -1003,7 +1005,8 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     }
     const size_t wide_bytes = (size_t)n_wide * kWideNodeFloat4 * 16;
     if (n_wide) {
-        e = arena_alloc(c, wide_bytes, &ds->arena_wide);
+        // the nodes, and their planes relative to the camera
+        e = arena_alloc(c, (kWideWidth == 4 ? 2 : 1) * wide_bytes, &ds->arena_wide);
         if (e != cudaSuccess) {
             ds->arena_wide = nullptr;
             release();
@@ -1011,6 +1014,12 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
                         cudaGetErrorString(e));
         }
         e = cudaMemcpyAsync(ds->arena_wide, h_wide, wide_bytes, cudaMemcpyHostToDevice, c->stream);
+        if (e == cudaSuccess && kWideWidth == 4) {
+            camera_basis(s->camera, ds->view.cam);
+            float4* w = static_cast<float4*>(ds->arena_wide);
+            e = launch_wide_relative(w, n_wide, ds->view.cam, w + (size_t)n_wide * kWideNodeFloat4,
+                                     c->stream);
+        }
         if (e != cudaSuccess) {
             release();
             return cuda_fail(c, e, "scene upload");
@@ -1037,6 +1046,7 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     SceneView& v = ds->view;
     v.nodes = reinterpret_cast<const float4*>(base + off_nodes);
     v.wide = n_wide ? static_cast<const float4*>(ds->arena_wide) : nullptr;
+    v.wide_cam = n_wide && kWideWidth == 4 ? v.wide + (size_t)n_wide * kWideNodeFloat4 : nullptr;
     v.geo_a = reinterpret_cast<const float4*>(base + off_ga);
     v.geo_b = reinterpret_cast<const float4*>(base + off_gb);
     v.geo_c = has_tri ? reinterpret_cast<const float4*>(base + off_gc) : nullptr;

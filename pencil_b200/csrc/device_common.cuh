@@ -716,6 +716,16 @@ __device__ __forceinline__ bool slab_nf(float nx, float ny, float nz, float fx, 
     return !(ex < en);
 }
 
+// The same with planes already relative to the ray's origin.
+__device__ __forceinline__ bool slab_rel(float nx, float ny, float nz, float fx, float fy,
+                                         float fz, const RayPre& r, float tmin, float tmax,
+                                         float& entry) {
+    const float en = fmax3f(fmaxf(tmin, nx * r.inv.x), ny * r.inv.y, nz * r.inv.z);
+    const float ex = fmin3f(fminf(tmax, fx * r.inv.x), fy * r.inv.y, fz * r.inv.z);
+    entry = en;
+    return !(ex < en);
+}
+
 __device__ __forceinline__ float f4c(const float4& v, int c) {
     return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w;
 }
@@ -724,9 +734,19 @@ __device__ __forceinline__ int i4c(const int4& v, int c) {
 }
 
 // Slab tests of every child: bit k of the result is child k's hit, e[k] its
-// entry distance.
+// entry distance. REL: the node's planes are relative to the ray's origin.
+template <bool REL = false>
 __device__ __forceinline__ unsigned slab_wide(const WideNode& w, const RayPre& r, float tmin,
                                               float tmax, float (&e)[kWideWidth]) {
+    if constexpr (REL && kWideWidth == 4) {
+        unsigned m = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            m |= slab_rel(f4c(w.nr[0][0], k), f4c(w.nr[1][0], k), f4c(w.nr[2][0], k),
+                          f4c(w.fr[0][0], k), f4c(w.fr[1][0], k), f4c(w.fr[2][0], k), r, tmin,
+                          tmax, e[k]) ? (1u << k) : 0u;
+        return m;
+    }
     unsigned m = 0;
     if constexpr (kWideWidth == 4) {
         m |= slab_nf(w.nr[0][0].x, w.nr[1][0].x, w.nr[2][0].x, w.fr[0][0].x, w.fr[1][0].x,

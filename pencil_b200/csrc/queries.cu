@@ -34,6 +34,32 @@ query_closest(SceneView S, const float* __restrict__ in, int n, int* __restrict_
     t_out[k] = slot >= 0 ? tb : -1.0f;
 }
 
+// wide_cam of a scene: every plane of the wide nodes minus the origin, refs as
+// they are. One thread per float4 row (4-wide nodes: rows 0-2 lo x y z, 3-5 hi).
+__global__ void __launch_bounds__(256)
+wide_relative(const float4* __restrict__ wide, long long rows, float ox, float oy, float oz,
+              float4* __restrict__ out) {
+    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (k >= rows) return;
+    float4 v = wide[k];
+    const int row = (int)(k & 7);
+    if (row < 6) {
+        const int a = row < 3 ? row : row - 3;
+        const float o = a == 0 ? ox : a == 1 ? oy : oz;
+        v = make_float4(v.x - o, v.y - o, v.z - o, v.w - o);
+    }
+    out[k] = v;
+}
+
+cudaError_t launch_wide_relative(const float4* wide, int n_wide, const float* origin, float4* out,
+                                 cudaStream_t st) {
+    const long long rows = (long long)n_wide * kWideNodeFloat4;
+    if (rows <= 0) return cudaSuccess;
+    wide_relative<<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(wide, rows, origin[0], origin[1],
+                                                                  origin[2], out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_query(const SceneView& S, bool camera, const float* in, int n, int* prim,
                          float* t, cudaStream_t st) {
     const int block = 128;

@@ -23,6 +23,8 @@
 //                               child has an empty box and a leaf ref of type
 //                               LEAF_NONE)
 //             [7G .. 8G)      = unused
+//   wide_cam                        the wide nodes again, with every plane minus
+//                                   the camera's origin (wf_camera)
 //   geo_a   float4[n_leaves]        leaf geometry in DFS leaf order (slot):
 //             sphere   (center.xyz, radius)
 //             triangle (v0.xyz, face normal x)
@@ -109,6 +111,9 @@ struct alignas(16) DevLight {
 struct SceneView {
     const float4* nodes;
     const float4* wide;    // wide nodes (null when the root is a leaf)
+    const float4* wide_cam;  // the same nodes, planes relative to the camera's
+                             // origin (camera rays share it): plane - origin,
+                             // rounded as the slab test rounds it
     const float4* geo_a;
     const float4* geo_b;
     const float4* geo_c;   // null in scenes without triangles

@@ -428,11 +428,17 @@ __device__ __forceinline__ void warp_append(bool take, int slot, int* counter, i
 // million paths of which 9 in 10 hit nothing: 27.4 -> 21.9 ms with this and
 // the list of shadow work that shade keeps; the sphere cloud's frame, whose
 // camera rays were written, read and shaded whether they hit or not, 24.44 ->
-// 24.11.)
+// 24.11.) The kernel is bound by the instructions it issues for each node, with
+// all lanes busy; camera rays share their origin, so it walks a copy of the
+// nodes whose planes the upload has taken the origin from, 24 subtractions a
+// node fewer (batch 17.4 -> 16.1 ms, sphere cloud 22.2 -> 21.8). Skipping the
+// reductions of children that are leaves cost more in branches than it saved
+// (batch 16.8).
 template <bool COUNT, bool ONE, bool KEEP>
 __global__ void __launch_bounds__(kWfMaxBlock) wf_camera(WfArgs A, long long path_begin, int n_slots) {
     __shared__ int s_ref[kWfMaxBlock / 32][kMaxStack];
     __shared__ float s_key[kWfMaxBlock / 32][kMaxStack];
+    constexpr bool REL = kWideWidth == 4;   // (the upload makes wide_cam for 4-wide nodes)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int* sref = s_ref[warp];
     float* skey = s_key[warp];
@@ -484,10 +490,10 @@ __global__ void __launch_bounds__(kWfMaxBlock) wf_camera(WfArgs A, long long pat
         if (__any_sync(0xffffffffu, active)) {
             int node = 0, sp = 0;
             while (true) {
-                const WideNode w = load_wide(S.wide, node, tr.rp);
+                const WideNode w = load_wide(REL ? S.wide_cam : S.wide, node, tr.rp);
                 if (COUNT && active) rc.tc.nodes++;
                 float ee[kWideWidth];
-                unsigned m = active ? slab_wide(w, tr.rp, tr.tmin, tr.t_best, ee) : 0u;
+                unsigned m = active ? slab_wide<REL>(w, tr.rp, tr.tmin, tr.t_best, ee) : 0u;
                 const unsigned lm = m & leaf_bits(w);
                 m &= ~lm;
                 unsigned ulm = __reduce_or_sync(0xffffffffu, lm);
