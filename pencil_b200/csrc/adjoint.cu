@@ -247,10 +247,11 @@ struct Replay {
                     if (l.kind == 2) continue;
                     int ns = (l.radius > 0.0f) ? P.soft : 1;
                     V3 ca = v3(0, 0, 0), ce = v3(0, 0, 0);
+                    const LightDisc disc = light_disc(l, h.p);
                     for (int k = 0; k < ns; ++k) {
                         V3 Ld;
                         float dist;
-                        light_dir(l, h.p, rng, Ld, dist);
+                        light_dir(l, disc, h.p, rng, Ld, dist);
                         if (glass) continue;
                         float ndotl = clampf(dot(h.n, Ld), 0.0f, 1.0f);
                         V3 phong = v3(0, 0, 0);

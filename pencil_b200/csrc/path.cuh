@@ -36,18 +36,32 @@ struct RayCount {
 };
 
 // Light direction and distance at p; soft point lights are jittered on a
-// disc facing p (src/renderer.hpp:512-545 and 887-906).
-__device__ __forceinline__ void light_dir(const DevLight& l, V3 p, Rng& rng, V3& L,
-                                          float& dist) {
-    V3 lp = ld3(l.pos);
+// disc facing p (src/renderer.hpp:512-545 and 887-906). The disc's axes are
+// the same for every sample of a vertex, and three normalizations (square
+// roots and divisions): a loop over samples takes them once (Whitted room of 63
+// primitives, 1.2M paths, four samples: 1.28 -> 1.20 ms; 64x64 tiles 4-5%
+// less), but in the wavefront's shading kernel (kDiscOnce), where the axes'
+// registers spill and path-traced frames pay for it (0.3%).
+struct LightDisc {
+    V3 t1, t2;
+};
+__device__ __forceinline__ LightDisc light_disc(const DevLight& l, V3 p) {
+    LightDisc f{v3(0, 0, 0), v3(0, 0, 0)};
     if (l.kind == 0 && l.radius > 0.0f) {
         V3 axis = normalized(ld3(l.pos) - p);
         V3 up = (fabsf(axis.y) < 0.9f) ? v3(0, 1, 0) : v3(1, 0, 0);
-        V3 t1 = normalized(cross(axis, up));
-        V3 t2 = normalized(cross(axis, t1));
+        f.t1 = normalized(cross(axis, up));
+        f.t2 = normalized(cross(axis, f.t1));
+    }
+    return f;
+}
+__device__ __forceinline__ void light_dir(const DevLight& l, const LightDisc& f, V3 p, Rng& rng,
+                                          V3& L, float& dist) {
+    V3 lp = ld3(l.pos);
+    if (l.kind == 0 && l.radius > 0.0f) {
         float dx, dy;
         rng.disc(dx, dy);
-        lp = ld3(l.pos) + (t1 * dx + t2 * dy) * l.radius;
+        lp = ld3(l.pos) + (f.t1 * dx + f.t2 * dy) * l.radius;
     }
     if (l.kind == 0) {
         V3 d = lp - p;
@@ -57,6 +71,10 @@ __device__ __forceinline__ void light_dir(const DevLight& l, V3 p, Rng& rng, V3&
         L = -ld3(l.pos);
         dist = 1e9f;
     }
+}
+__device__ __forceinline__ void light_dir(const DevLight& l, V3 p, Rng& rng, V3& L,
+                                          float& dist) {
+    light_dir(l, light_disc(l, p), p, rng, L, dist);
 }
 
 // Contribution of a visible point/directional light sample at a path-trace
@@ -294,10 +312,13 @@ __device__ __forceinline__ bool shade_vertex(const SceneView& S, const PathParam
             const DevLight& l = S.lights[li];
             if (l.kind == 2) continue;
             int ns = (l.radius > 0.0f) ? P.soft : 1;
+            LightDisc disc{};
+            if (Emit::kDiscOnce) disc = light_disc(l, h.p);
             for (int k = 0; k < ns; ++k) {
                 V3 L;
                 float dist;
-                light_dir(l, h.p, ps.rng, L, dist);
+                if (!Emit::kDiscOnce) disc = light_disc(l, h.p);
+                light_dir(l, disc, h.p, ps.rng, L, dist);
                 if (glass) continue;
                 float ndotl = clampf(dot(h.n, L), 0.0f, 1.0f);
                 V3 c = albedo * ld3(l.intensity) * ndotl;
@@ -423,10 +444,11 @@ struct Tracer {
             if (l.kind == 2) continue;
             V3 contrib = v3(0, 0, 0);
             int ns = (l.radius > 0.0f) ? P.soft : 1;
+            const LightDisc disc = light_disc(l, h.p);
             for (int k = 0; k < ns; ++k) {
                 V3 L;
                 float dist;
-                light_dir(l, h.p, rng, L, dist);
+                light_dir(l, disc, h.p, rng, L, dist);
                 if (!shade) continue;
                 Ray sr{h.p + h.n * P.bias, L};
                 float ndotl = clampf(dot(h.n, L), 0.0f, 1.0f);
@@ -478,10 +500,11 @@ struct Tracer {
             const DevLight& l = S.lights[li];
             if (l.kind == 2) continue;
             const int ns = (l.radius > 0.0f) ? P.soft : 1;
+            const LightDisc disc = light_disc(l, h.p);
             for (int k = 0; k < ns; ++k) {
                 V3 L;
                 float dist;
-                light_dir(l, h.p, rng, L, dist);
+                light_dir(l, disc, h.p, rng, L, dist);
                 put(t, L, dist - P.bias, 0.0f, li, k == ns - 1 ? ns : 0);
                 if (t.n == team) drain(t, sorg, term, add);
             }
@@ -720,6 +743,7 @@ struct Tracer {
 
     // Shadow rays of one vertex traced as they are made.
     struct InlineNee {
+        static constexpr bool kDiscOnce = true;
         Tracer& tr;
         NeeAccum acc;
         V3 tail, w;

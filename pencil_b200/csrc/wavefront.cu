@@ -586,6 +586,7 @@ __global__ void __launch_bounds__(kWfMaxBlock) wf_camera(WfArgs A, long long pat
 // untested, for the ends of its lights' groups).
 template <bool SKIP>
 struct StoreNee {
+    static constexpr bool kDiscOnce = false;
     const WfArgs& A;
     int slot;
     int n;
