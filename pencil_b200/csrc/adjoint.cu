@@ -102,7 +102,8 @@ __device__ __forceinline__ void flush_contrib(bool has, int key, V3 v, double* g
 
 // FOUND: hits and visibility come from a wavefront pass instead of rays traced
 // here.
-template <bool COUNT, bool FOUND>
+// VARIANT: one per kernel, so that each has its own copy to inline.
+template <bool COUNT, bool FOUND, int VARIANT>
 struct Replay {
     const SceneView& S;
     const PathParams& P;
@@ -314,9 +315,14 @@ struct Replay {
 // in local memory either way, and the extra resident warps hide more of its
 // latency (per gradient: 16.45 ms; 17.49 at 80 registers, 16.70 at 64).
 constexpr int kAdjMinBlocks = 7;
+// A launch of one wave at four blocks per SM waits for its longest paths, not
+// for issue slots, and gets 128 registers (12,288 paths 0.203 -> 0.191 ms; 76,800,
+// just beyond the line, would gain 0.53 -> 0.47, 120,000 lose 0.67 -> 0.71).
+constexpr int kAdjSmallBlocks = 4;
+constexpr long long kAdjSmallThreads = 148LL * kAdjSmallBlocks * kAdjBlock;
 
-template <bool COUNT, bool FOUND>
-__global__ void __launch_bounds__(kAdjBlock, kAdjMinBlocks)
+template <bool COUNT, bool FOUND, int MINB>
+__global__ void __launch_bounds__(kAdjBlock, MINB)
 adjoint_kernel(AdjArgs A) {
     extern __shared__ int smem[];
     TravStack<kAdjShared> stk;
@@ -327,7 +333,7 @@ adjoint_kernel(AdjArgs A) {
     }
     RayCount rc = {};
     const PathParams& P = A.P;
-    Replay<COUNT, FOUND> rp{A.S, P, stk, rc, A.found, 0, 0};
+    Replay<COUNT, FOUND, MINB> rp{A.S, P, stk, rc, A.found, 0, 0};
     const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long pix = A.pix_begin + gid / A.G;
     const int lane_g = (int)(gid % A.G);
@@ -450,8 +456,12 @@ cudaError_t launch_adjoint(const SceneView& S, const RenderCfg& c, const Adjoint
     A.pix_end = (long long)c.W * c.H;
     const size_t smem = (size_t)kAdjShared * kAdjBlock * 8;
     const unsigned blocks = adjoint_blocks(A);
-    if (c.count) adjoint_kernel<true, false><<<blocks, kAdjBlock, smem, st>>>(A);
-    else adjoint_kernel<false, false><<<blocks, kAdjBlock, smem, st>>>(A);
+    if (c.count)
+        adjoint_kernel<true, false, kAdjMinBlocks><<<blocks, kAdjBlock, smem, st>>>(A);
+    else if (A.pix_end * A.G <= kAdjSmallThreads)
+        adjoint_kernel<false, false, kAdjSmallBlocks><<<blocks, kAdjBlock, smem, st>>>(A);
+    else
+        adjoint_kernel<false, false, kAdjMinBlocks><<<blocks, kAdjBlock, smem, st>>>(A);
     return cudaGetLastError();
 }
 
@@ -462,7 +472,7 @@ cudaError_t launch_adjoint_found(const SceneView& S, const RenderCfg& c, const A
     A.found = AdjFound{hit, vis, stride, pix_begin * c.spp};
     A.pix_begin = pix_begin;
     A.pix_end = pix_begin + pixels;
-    adjoint_kernel<false, true><<<adjoint_blocks(A), kAdjBlock, 0, st>>>(A);
+    adjoint_kernel<false, true, kAdjMinBlocks><<<adjoint_blocks(A), kAdjBlock, 0, st>>>(A);
     return cudaGetLastError();
 }
 

@@ -159,3 +159,20 @@ def test_automatic_capacity_over_frames_of_many_shapes(gpu):
     ctx.close()
     gpu.free(a)
     gpu.free(b)
+
+
+@pytest.mark.parametrize("size", [(148, 1024, 1), (151553, 1, 1), (296, 128, 2), (37889, 1, 2)])
+@pytest.mark.parametrize("name,pathtrace", [("cloud2k", True), ("prims_mix", False)])
+def test_register_budgets_render_the_same_image(gpu, size, name, pathtrace):
+    """151,552 threads, the most that the kernel with four blocks per SM is
+    launched for, and one pixel more: the counting kernel's image."""
+    scene, _ = load_golden(name)
+    sid = gpu.upload(scene)
+    w, h, n = size
+    st = RenderSettings(width=w, height=h, samples=n, max_depth=4, pathtrace=pathtrace,
+                        pathtrace_bounces=4, engine=A.ENGINE_MEGAKERNEL)
+    m2 = [np.empty((h, w, 3), np.float32) for _ in range(2)]
+    a = gpu.render(sid, st, None, m2[0])
+    b = gpu.render(sid, dataclasses.replace(st, count_rays=True), None, m2[1])
+    assert np.array_equal(a, b) and np.array_equal(m2[0], m2[1])
+    gpu.free(sid)
