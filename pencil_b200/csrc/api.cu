@@ -30,6 +30,7 @@ cudaError_t launch_query(const SceneView& S, bool camera, const float* in, int n
 
 struct WfScratch;
 WfScratch* wavefront_new();
+void wavefront_release(WfScratch& W);
 void wavefront_delete(WfScratch* W);
 cudaError_t wavefront_render(WfScratch& W, const std::vector<SceneView>& views,
                              const std::vector<std::vector<DevLight>>& lights,
@@ -276,6 +277,12 @@ cudaError_t ensure_pool(pgpu_ctx* c) {
 cudaError_t arena_alloc(pgpu_ctx* c, size_t bytes, void** out) {
     cudaError_t e = ensure_pool(c);
     if (e != cudaSuccess) return e;
+    e = cudaMallocFromPoolAsync(out, bytes, c->pool, c->stream);
+    if (e != cudaErrorMemoryAllocation) return e;
+    // the renders' scratch makes room: the next render takes what is left
+    (void)cudaGetLastError();
+    if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return e;
+    wavefront_release(*c->wf);
     return cudaMallocFromPoolAsync(out, bytes, c->pool, c->stream);
 }
 
@@ -1004,9 +1011,16 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
                     wide_stack, kMaxDepth);
     }
     const size_t wide_bytes = (size_t)n_wide * kWideNodeFloat4 * 16;
+    bool relative = false;
     if (n_wide) {
-        // the nodes, and their planes relative to the camera
-        e = arena_alloc(c, (kWideWidth == 4 ? 2 : 1) * wide_bytes, &ds->arena_wide);
+        // the nodes, and their planes relative to the camera where both fit
+        // (without, camera rays are traced one per lane)
+        if (kWideWidth == 4) {
+            e = arena_alloc(c, 2 * wide_bytes, &ds->arena_wide);
+            relative = e == cudaSuccess;
+            if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
+        }
+        if (!relative) e = arena_alloc(c, wide_bytes, &ds->arena_wide);
         if (e != cudaSuccess) {
             ds->arena_wide = nullptr;
             release();
@@ -1014,7 +1028,7 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
                         cudaGetErrorString(e));
         }
         e = cudaMemcpyAsync(ds->arena_wide, h_wide, wide_bytes, cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess && kWideWidth == 4) {
+        if (e == cudaSuccess && relative) {
             camera_basis(s->camera, ds->view.cam);
             float4* w = static_cast<float4*>(ds->arena_wide);
             e = launch_wide_relative(w, n_wide, ds->view.cam, w + (size_t)n_wide * kWideNodeFloat4,
@@ -1046,7 +1060,7 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     SceneView& v = ds->view;
     v.nodes = reinterpret_cast<const float4*>(base + off_nodes);
     v.wide = n_wide ? static_cast<const float4*>(ds->arena_wide) : nullptr;
-    v.wide_cam = n_wide && kWideWidth == 4 ? v.wide + (size_t)n_wide * kWideNodeFloat4 : nullptr;
+    v.wide_cam = relative ? v.wide + (size_t)n_wide * kWideNodeFloat4 : nullptr;
     v.geo_a = reinterpret_cast<const float4*>(base + off_ga);
     v.geo_b = reinterpret_cast<const float4*>(base + off_gb);
     v.geo_c = has_tri ? reinterpret_cast<const float4*>(base + off_gc) : nullptr;

@@ -1168,6 +1168,12 @@ static int max_shadow_records(const SceneView& v, const std::vector<DevLight>& l
 
 static cudaError_t ensure_streams(WfScratch& W);
 
+// Camera packets walk the camera-relative nodes, which an upload short of
+// memory leaves out.
+static bool packets_for(const SceneView& v) {
+    return kWideWidth != 4 || !v.wide || v.wide_cam;
+}
+
 struct WfOccupancy {
     int grid_extend = 0, grid_shade = 0, grid_shadow = 0, grid_scatter = 0, grid_packet = 0;
     int grid_accumulate = 0;
@@ -1390,7 +1396,7 @@ cudaError_t wavefront_render(WfScratch& W, const std::vector<SceneView>& views,
         sort_key = c.sort_key;
         if (c.refill > 0) refill = c.refill;
         if (c.block > 0) block = c.block;
-        packets = packets && c.packets;
+        packets = packets && c.packets && packets_for(views[J.view]);
     }
     total_paths = path_off;
     // Fault injection, host side: PGPU_INJECT_SHADOW_RECORDS=k gives every
@@ -1580,7 +1586,8 @@ cudaError_t wavefront_adjoint(WfScratch& W, const SceneView& view,
     *done = false;
     const long long paths = cfg.pixels() * cfg.spp;
     const int maxS = max_shadow_records(view, lights, cfg.soft);
-    if (cfg.count || cfg.depth < 1 || maxS > 32 || paths <= kAdjOneKernel || cfg.spp > kAdjChunk)
+    if (!packets_for(view) || cfg.count || cfg.depth < 1 || maxS > 32 || paths <= kAdjOneKernel ||
+        cfg.spp > kAdjChunk)
         return cudaSuccess;
     const long long ppc = std::min<long long>(kAdjChunk / cfg.spp, cfg.pixels());
     const int Q = (int)(ppc * cfg.spp);
