@@ -1251,7 +1251,8 @@ int make_cfg(pgpu_ctx* c, const DeviceScene* ds, const pgpu_render_params* p, Re
     cfg.profile = (p->flags & PGPU_FLAG_PROFILE_KERNELS) != 0;
     cfg.packets = (p->flags & PGPU_FLAG_NO_PACKETS) == 0;
     cfg.mis = (p->flags & PGPU_FLAG_MIS) != 0;
-    cfg.binary_tree = (p->flags & PGPU_FLAG_BINARY_TREE) != 0;
+    // (the queues walk the wide tree, and so does a frame of theirs in one kernel)
+    cfg.binary_tree = cfg.engine == PGPU_ENGINE_MEGAKERNEL && (p->flags & PGPU_FLAG_BINARY_TREE);
     if (p->block_size != 0 && p->block_size != 64 && p->block_size != 128 && p->block_size != 256)
         return fail(c, PGPU_ERR_INVALID_ARG, "block_size must be 0, 64, 128 or 256");
     cfg.block = p->block_size;
