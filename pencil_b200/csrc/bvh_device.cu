@@ -866,11 +866,12 @@ sah_local(const SahTask* local, const int* n_local, int* perm, const DBox* boxes
                         }
                     }
                 }
-                // the first of the cheapest boundaries (costs are at least 1)
-                const unsigned least = __reduce_min_sync(all, __float_as_uint(cost));
-                const bool split = __uint_as_float(least) < FLT_MAX;
+                // the first of the cheapest boundaries (below zero where a side
+                // holds only boxes with a NaN plane)
+                const int least = __reduce_min_sync(all, ord(cost));
+                const bool split = least < ord(FLT_MAX);
                 if (split) {
-                    const int best = __ffs(__ballot_sync(all, __float_as_uint(cost) == least)) - 1;
+                    const int best = __ffs(__ballot_sync(all, ord(cost) == least)) - 1;
                     nl = __shfl_sync(all, nl, best);
                     for (int a = 0; a < 3; ++a) {
                         lb.mn[a] = __shfl_sync(all, lb.mn[a], best);
@@ -894,34 +895,39 @@ sah_local(const SahTask* local, const int* n_local, int* perm, const DBox* boxes
                     }
                 } else {
                     // median split: each primitive's place in the stable order
-                    // by centroid sum
+                    // by centroid sum. The keys are compared as their ord()
+                    // images, of which no two are unordered: a box that is not
+                    // finite has a NaN key, and every place must be taken once
+                    // (+ 0.0f: the two zeros tie). NaN planes go into the sides'
+                    // boxes in the same order.
                     nl = count / 2;
-                    for (int a = 0; a < 3; ++a) {
-                        lb.mn[a] = rb.mn[a] = 1e30f;
-                        lb.mx[a] = rb.mx[a] = -1e30f;
-                    }
+                    int lo[2][3], hi[2][3];
+                    for (int h = 0; h < 2; ++h)
+                        for (int a = 0; a < 3; ++a) { lo[h][a] = ord(1e30f); hi[h][a] = ord(-1e30f); }
                     for (int i = lane; i < count; i += 32) {
                         const int q = s_perm[off + i];
-                        const float key = sah_key2(s_box[q], axis);
+                        const int key = ord(sah_key2(s_box[q], axis) + 0.0f);
                         int rank = 0;
                         for (int j = 0; j < count; ++j) {
-                            const float kj = sah_key2(s_box[s_perm[off + j]], axis);
+                            const int kj = ord(sah_key2(s_box[s_perm[off + j]], axis) + 0.0f);
                             rank += (kj < key || (kj == key && j < i)) ? 1 : 0;
                         }
                         s_tmp[off + rank] = q;
-                        DBox& d = rank < nl ? lb : rb;
+                        const bool right = rank >= nl;
                         for (int a = 0; a < 3; ++a) {
-                            d.mn[a] = fminf(d.mn[a], s_box[q].mn[a]);
-                            d.mx[a] = fmaxf(d.mx[a], s_box[q].mx[a]);
+                            const int mn = ord(s_box[q].mn[a]), mx = ord(s_box[q].mx[a]);
+                            lo[0][a] = min(lo[0][a], right ? INT_MAX : mn);
+                            hi[0][a] = max(hi[0][a], right ? INT_MIN : mx);
+                            lo[1][a] = min(lo[1][a], right ? mn : INT_MAX);
+                            hi[1][a] = max(hi[1][a], right ? mx : INT_MIN);
                         }
                     }
-                    for (int o = 16; o > 0; o >>= 1)
-                        for (int a = 0; a < 3; ++a) {
-                            lb.mn[a] = fminf(lb.mn[a], __shfl_xor_sync(all, lb.mn[a], o));
-                            lb.mx[a] = fmaxf(lb.mx[a], __shfl_xor_sync(all, lb.mx[a], o));
-                            rb.mn[a] = fminf(rb.mn[a], __shfl_xor_sync(all, rb.mn[a], o));
-                            rb.mx[a] = fmaxf(rb.mx[a], __shfl_xor_sync(all, rb.mx[a], o));
-                        }
+                    for (int a = 0; a < 3; ++a) {
+                        lb.mn[a] = unord(__reduce_min_sync(all, lo[0][a]));
+                        lb.mx[a] = unord(__reduce_max_sync(all, hi[0][a]));
+                        rb.mn[a] = unord(__reduce_min_sync(all, lo[1][a]));
+                        rb.mx[a] = unord(__reduce_max_sync(all, hi[1][a]));
+                    }
                 }
                 __syncwarp();
                 for (int i = lane; i < count; i += 32) s_perm[off + i] = s_tmp[off + i];

@@ -214,3 +214,158 @@ def test_device_sah_subtrees_built_by_one_block(gpu, n, kind):
     if kind == "random":
         host, host_depth = s.build_bvh()
         assert depth == host_depth and np.array_equal(nodes, host)
+
+
+# ---- primitives that are not finite ------------------------------------------------
+# pgpu_build_bvh_device* take any bits (an upload does not): the table must
+# still hold every primitive once.
+
+def _ord(f):
+    """The int image that orders floats as their bits do; NaN as the device makes it."""
+    i = np.where(np.isnan(f), np.int32(0x7fffffff), np.asarray(f, np.float32).view(np.int32))
+    return np.where(i >= 0, i, i ^ np.int32(0x7fffffff)).astype(np.int32)
+
+
+def _unord(i):
+    i = np.asarray(i, np.int32)
+    return np.where(i >= 0, i, i ^ np.int32(0x7fffffff)).astype(np.int32).view(np.float32)
+
+
+def _ord_box(mn, mx):
+    """Bounds of boxes by bit order: a NaN plane is the largest."""
+    return (_unord(np.minimum(_ord(mn).min(0), _ord(np.float32(1e30)))),
+            _unord(np.maximum(_ord(mx).max(0), _ord(np.float32(-1e30)))))
+
+
+def _axis(mn, mx):
+    e = mx - mn
+    return 0 if e[0] >= e[1] and e[0] >= e[2] else 1 if e[1] >= e[2] else 2
+
+
+def _area(mn, mx):
+    e = mx - mn
+    return np.float32(2) * (e[0] * e[1] + e[1] * e[2] + e[0] * e[2])
+
+
+def sah_model(mn, mx):
+    """The device's SAH build over boxes of any bits, one node at a time."""
+    F = np.float32
+    n = len(mn)
+    out = np.zeros(2 * n - 1, A.NODE_DTYPE)
+    empty = (np.full(3, 1e30, F), np.full(3, -1e30, F))
+
+    def write(at, box, left, right):
+        out[at] = (box[0], left, box[1], right)
+
+    def small(items, node):
+        lo, hi = (np.fmin.reduce(np.vstack([empty[0][None], mn[items]])),
+                  np.fmax.reduce(np.vstack([empty[1][None], mx[items]])))
+        if len(items) == 1:
+            return write(node, (lo, hi), -1, items[0])
+        a = _axis(lo, hi)
+        items = list(items)
+        for i in range(1, len(items)):
+            v, j = items[i], i - 1
+            while j >= 0 and mn[items[j], a] + mx[items[j], a] > mn[v, a] + mx[v, a]:
+                items[j + 1] = items[j]
+                j -= 1
+            items[j + 1] = v
+        h = len(items) // 2
+        write(node, (lo, hi), node + 1, node + 2 * h)
+        small(items[:h], node + 1)
+        small(items[h:], node + 2 * h)
+
+    def build(items, node, box):
+        if len(items) == 1:
+            return write(node, box, -1, items[0])
+        if len(items) <= 4:
+            return small(items, node)
+        a = _axis(*box)
+        best, cut, sides = np.finfo(F).max, 0, None
+        if box[1][a] > box[0][a]:
+            f = ((mn[items, a] + mx[items, a]) * F(0.5) - box[0][a]) / (box[1][a] - box[0][a]) * F(12)
+            k = np.nan_to_num(f, nan=0.0, posinf=12.0, neginf=0.0).clip(0, 11).astype(int)
+            bins = [_ord_box(mn[items[k == q]], mx[items[k == q]]) if (k == q).any() else empty
+                    for q in range(12)]
+            sa = _area(*box)
+            for b in range(1, 12):
+                nl = int((k < b).sum())
+                if nl == 0 or nl == len(items):
+                    continue
+                half = [(np.fmin.reduce([empty[0]] + [x[0] for x in part]),
+                         np.fmax.reduce([empty[1]] + [x[1] for x in part]))
+                        for part in (bins[:b], bins[b:])]
+                cost = F(1) + (F(nl) * _area(*half[0]) + F(len(items) - nl) * _area(*half[1])) / \
+                    (sa if sa > 0 else F(1))
+                if cost < best:
+                    best, cut, sides = cost, b, half
+        if cut:
+            left, right = items[k < cut], items[k >= cut]
+        else:
+            order = items[np.argsort(_ord(mn[items, a] + mx[items, a] + F(0)), kind="stable")]
+            left, right = order[:len(items) // 2], order[len(items) // 2:]
+            sides = [_ord_box(mn[p], mx[p]) for p in (left, right)]
+        write(node, box, node + 1, node + 2 * len(left))
+        build(left, node + 1, sides[0])
+        build(right, node + 2 * len(left), sides[1])
+
+    with np.errstate(all="ignore"):
+        if n > 4:
+            build(np.arange(n), 0, (_unord(_ord(mn).min(0)), _unord(_ord(mx).max(0))))
+        else:
+            small(np.arange(n), 0)
+    return out
+
+
+def leaves_once(nodes, n):
+    """Links of a DFS table, and every primitive in one leaf (boxes aside)."""
+    plain = nodes.copy()
+    plain["bmin"], plain["bmax"] = 0, 0
+    return check_table(plain, n)
+
+
+@pytest.mark.parametrize("n", [5, 7, 33, 512, 513, 1500])
+@pytest.mark.parametrize("kind", ["nan", "nan_axis", "inf", "all_nan", "half_nan_point"])
+def test_device_builds_of_primitives_that_are_not_finite(gpu, n, kind):
+    from pencil_b200.scene import Material, Scene
+    rng = np.random.default_rng(n)
+    c = rng.uniform(-10, 10, (n, 3)).astype(np.float32)
+    r = rng.uniform(0.01, 0.3, n).astype(np.float32)
+    if kind == "nan":
+        c[rng.choice(n, max(n // 10, 1), replace=False)] = np.nan
+    elif kind == "nan_axis":
+        for a in range(3):
+            c[rng.choice(n, max(n // 20, 1), replace=False), a] = np.nan
+    elif kind == "inf":
+        r[rng.choice(n, max(n // 10, 1), replace=False)] = np.inf
+        c[0] = (-np.inf, np.inf, 0)
+    elif kind == "all_nan":
+        c[:] = np.nan
+    else:
+        c[:] = c[0]
+        c[::2] = np.nan
+    s = Scene()
+    m = s.add_material(Material.diffuse((1, 1, 1)))
+    s.add_spheres(c, r, np.full(n, m, np.int32))
+    nodes, depth = gpu.build_bvh_device(s, "sah")
+    assert leaves_once(nodes, n) == depth
+    with np.errstate(all="ignore"):
+        want = sah_model(c - r[:, None], c + r[:, None])
+    assert np.array_equal(nodes["left"], want["left"])
+    assert np.array_equal(nodes["right"], want["right"])
+    assert np.array_equal(nodes["bmin"], want["bmin"], equal_nan=True)
+    assert np.array_equal(nodes["bmax"], want["bmax"], equal_nan=True)
+    nodes, depth = gpu.build_bvh_device(s, "lbvh")
+    assert leaves_once(nodes, n) == depth
+
+
+def test_device_builds_of_a_mesh_with_broken_vertices(gpu):
+    w = W.mesh_box(4, 8, 8, 1, 1)
+    s, rng = w.scene, np.random.default_rng(3)
+    v = s.mesh_vertices.copy()
+    v[rng.choice(len(v), len(v) // 20, replace=False)] = np.nan
+    v[rng.choice(len(v), len(v) // 20, replace=False), 1] = np.inf
+    s.set_mesh(v, s.mesh_indices, s.mesh_materials)
+    for method in ("sah", "lbvh"):
+        nodes, depth = gpu.build_bvh_device(s, method)
+        assert leaves_once(nodes, s.n_unified) == depth
