@@ -757,7 +757,8 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
         std::memcpy(d.pos, l.pos, 12);
         std::memcpy(d.intensity, l.intensity, 12);
         d.radius = l.radius;
-        d.is_emissive = l.is_emissive;
+        // (a quad's visibility is tested whatever the flag says)
+        d.is_emissive = l.kind == PGPU_LIGHT_QUAD ? 0 : l.is_emissive;
         std::memcpy(d.edge_u, l.edge_u, 12);
         std::memcpy(d.edge_v, l.edge_v, 12);
         if (l.kind == PGPU_LIGHT_QUAD) {

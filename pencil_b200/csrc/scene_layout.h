@@ -99,7 +99,7 @@ struct alignas(16) DevLight {
     float pos[3];
     float intensity[3];
     float radius;
-    int is_emissive;
+    int is_emissive;       // no shadow test (0 for quads)
     float edge_u[3];
     float edge_v[3];
     float area;            // quad: |edge_u x edge_v|

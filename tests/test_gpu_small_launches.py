@@ -176,3 +176,35 @@ def test_register_budgets_render_the_same_image(gpu, size, name, pathtrace):
     b = gpu.render(sid, dataclasses.replace(st, count_rays=True), None, m2[1])
     assert np.array_equal(a, b) and np.array_equal(m2[0], m2[1])
     gpu.free(sid)
+
+
+@pytest.mark.parametrize("pathtrace", [False, True])
+def test_quad_lights_are_tested_whatever_their_flag(gpu, pathtrace):
+    """is_emissive is the point and directional lights' way past the shadow
+    test; a quad light that sets it is shadowed all the same: in the
+    reference-exact groups, in one kernel, on the queues, and in gradients of
+    both kinds."""
+    out = []
+    for flag in (False, True):
+        scene, _ = load_golden("prims_mix")
+        lamp = Light.quad((-1, 6, -1), (1, 0, 0), (0, 0, 1), (9, 9, 9), 1)
+        scene.add_light(dataclasses.replace(lamp, is_emissive=flag))
+        sid = gpu.upload(scene)
+        st = RenderSettings(width=64, height=48, samples=2, max_depth=4, pathtrace=pathtrace,
+                            pathtrace_bounces=4)
+        exact = dict(engine=A.ENGINE_MEGAKERNEL, rng=A.RNG_PIXEL_SEQUENTIAL,
+                     glass=A.GLASS_BOTH_BRANCHES)
+        got = [gpu.render(sid, dataclasses.replace(st, **kw))
+               for kw in (exact, dict(exact, binary_tree=True), dict(), dict(block_size=128),
+                          dict(count_rays=True))]
+        for w, h in ((64, 48), (300, 240)):
+            dl = np.random.default_rng(1).normal(size=(h, w, 3)).astype(np.float32)
+            got += gpu.adjoint(sid, dataclasses.replace(st, width=w, height=h), dl,
+                               scene.n_materials, len(scene.lights), want_image=True)
+        out.append(got)
+        gpu.free(sid)
+    for a, b in zip(*out):
+        if a.dtype == np.float32:
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+        else:                       # FP64 sums in another order
+            assert np.abs(a - b).max() <= 1e-9 * max(np.abs(b).max(), 1e-30)
