@@ -31,6 +31,7 @@
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "host_internal.h"
@@ -1049,15 +1050,11 @@ static int lanes_for(int spp) {
     return G;
 }
 
-// Scratch of the wavefront, owned by the context (grown on demand).
+// Scratch of the wavefront, owned by the context: one block, as large as the
+// largest frame so far needed, that every frame lays out for its own shape.
 struct WfScratch {
     void* mem = nullptr;
     size_t bytes = 0;
-    int Q = 0;
-    int maxS = 0;
-    int iters = 0;
-    int jobs_cap = 0;
-    int views_cap = 0;
     int block = kWfBlock;             // threads per block of this frame's kernels
     WfArgs args{};
     SceneView* d_views = nullptr;
@@ -1078,79 +1075,78 @@ struct WfScratch {
 
 static size_t al(size_t x) { return (x + 255) & ~size_t(255); }
 
-static cudaError_t ensure_scratch(WfScratch& W, int Q, int maxS, int iters, int n_jobs,
-                                  int n_views) {
-    if (W.mem && W.Q >= Q && W.maxS >= maxS && W.iters >= iters && W.jobs_cap >= n_jobs &&
-        W.views_cap >= n_views)
-        return cudaSuccess;
-    if (W.graph) { cudaGraphExecDestroy(W.graph); W.graph = nullptr; W.graph_key = 0; }
-    if (W.mem) cudaFree(W.mem);
-    W.mem = nullptr;
-    // room for the earlier frames' shapes as well, unless many paths of one and
-    // many records of another would multiply beyond 16 GiB
-    if ((long long)std::max(Q, W.Q) * (212 + 64LL * std::max(maxS, W.maxS)) <= 16LL << 30) {
-        Q = std::max(Q, W.Q);
-        maxS = std::max(maxS, W.maxS);
-    }
-    maxS = std::max(maxS, 1);
-    iters = std::max(iters, W.iters);
-    n_jobs = std::max(n_jobs, W.jobs_cap);
-    n_views = std::max(n_views, W.views_cap);
-    size_t per = al((size_t)Q * 16);
-    size_t sz = 0;
-    sz += 8 * per;                                   // ray_o ray_d T L st hit pb pw
-    sz += 4 * (size_t)maxS * per;                    // shadow records (64 B each)
-    sz += 2 * al((size_t)kOctants * Q * 4);          // queues
-    sz += al((size_t)(iters + 2) * kOctants * 4);    // counts
-    sz += al((size_t)(iters + 2) * 3 * 4);           // work cursors
-    sz += al(4);                                     // status
-    sz += 5 * al((size_t)Q * 4);                     // sort: keys, list, sorted queues
-    sz += al((size_t)kSortBins * 4) + al((size_t)kSortBinsE * 4);        // sort: histograms
-    sz += al((size_t)kSortChunks * 4) + al((size_t)kSortChunksE * 4);    // chunk offsets
-    sz += al((size_t)(iters + 2) * 2 * 4);           // sort: list counts
-    sz += al((size_t)n_views * sizeof(SceneView));
-    sz += al((size_t)n_jobs * sizeof(WfJob));
-    cudaError_t e = cudaMalloc(&W.mem, sz);
-    if (e != cudaSuccess) { W.mem = nullptr; W.bytes = 0; W.Q = 0; return e; }
-    W.bytes = sz;
-    W.Q = Q;
-    W.maxS = maxS;
-    W.iters = iters;
-    W.jobs_cap = n_jobs;
-    W.views_cap = n_views;
-    unsigned char* p = static_cast<unsigned char*>(W.mem);
-    auto take = [&](size_t b) { unsigned char* r = p; p += al(b); return r; };
+// Lays out the arrays of a frame's shape from `base` in W.args, W.d_views and
+// W.d_jobs; returns the bytes they take.
+static size_t carve(WfScratch& W, void* base, int Q, int maxS, int iters, int n_jobs,
+                    int n_views) {
+    size_t used = 0;
+    auto take = [&](auto*& ptr, size_t count) {
+        using T = std::remove_reference_t<decltype(*ptr)>;
+        ptr = reinterpret_cast<T*>(static_cast<unsigned char*>(base) + used);
+        used += al(count * sizeof(T));
+    };
     WfArgs& A = W.args;
+    const size_t q = (size_t)Q, levels = (size_t)iters + 2;
     A.Q = Q;
     A.maxS = maxS;
-    A.ray_o = reinterpret_cast<float4*>(take((size_t)Q * 16));
-    A.ray_d = reinterpret_cast<float4*>(take((size_t)Q * 16));
-    A.T = reinterpret_cast<float4*>(take((size_t)Q * 16));
-    A.L = reinterpret_cast<float4*>(take((size_t)Q * 16));
-    A.st = reinterpret_cast<uint4*>(take((size_t)Q * 16));
-    A.hit = reinterpret_cast<float4*>(take((size_t)Q * 16));
-    A.pb = reinterpret_cast<float4*>(take((size_t)Q * 16));
-    A.pw = reinterpret_cast<float4*>(take((size_t)Q * 16));
-    A.rec = reinterpret_cast<float4*>(take((size_t)maxS * Q * 64));
-    A.q[0] = reinterpret_cast<int*>(take((size_t)kOctants * Q * 4));
-    A.q[1] = reinterpret_cast<int*>(take((size_t)kOctants * Q * 4));
-    A.counts = reinterpret_cast<int*>(take((size_t)(iters + 2) * kOctants * 4));
-    A.work = reinterpret_cast<unsigned int*>(take((size_t)(iters + 2) * 3 * 4));
-    A.status = reinterpret_cast<int*>(take(4));
-    A.key_s = reinterpret_cast<int*>(take((size_t)Q * 4));
-    A.tmp_s = reinterpret_cast<int*>(take((size_t)Q * 4));
-    A.qs = reinterpret_cast<int*>(take((size_t)Q * 4));
-    A.hist_s = reinterpret_cast<int*>(take((size_t)kSortBins * 4));
-    A.chunk_off = reinterpret_cast<int*>(take((size_t)kSortChunks * 4));
-    A.key_e = reinterpret_cast<int*>(take((size_t)Q * 4));
-    A.qe = reinterpret_cast<int*>(take((size_t)Q * 4));
-    A.hist_e = reinterpret_cast<int*>(take((size_t)kSortBinsE * 4));
-    A.chunk_off_e = reinterpret_cast<int*>(take((size_t)kSortChunksE * 4));
-    A.tcnt = reinterpret_cast<int*>(take((size_t)(iters + 2) * 2 * 4));
-    W.d_views = reinterpret_cast<SceneView*>(take((size_t)n_views * sizeof(SceneView)));
-    W.d_jobs = reinterpret_cast<WfJob*>(take((size_t)n_jobs * sizeof(WfJob)));
+    take(A.ray_o, q);
+    take(A.ray_d, q);
+    take(A.T, q);
+    take(A.L, q);
+    take(A.st, q);
+    take(A.hit, q);
+    take(A.pb, q);
+    take(A.pw, q);
+    take(A.rec, 4 * (size_t)maxS * q);        // 64 bytes a shadow record
+    take(A.q[0], kOctants * q);
+    take(A.q[1], kOctants * q);
+    take(A.counts, levels * kOctants);
+    take(A.work, levels * 3);
+    take(A.status, 1);
+    take(A.key_s, q);
+    take(A.tmp_s, q);
+    take(A.qs, q);
+    take(A.hist_s, kSortBins);
+    take(A.chunk_off, kSortChunks);
+    take(A.key_e, q);
+    take(A.qe, q);
+    take(A.hist_e, kSortBinsE);
+    take(A.chunk_off_e, kSortChunksE);
+    take(A.tcnt, levels * 2);
+    take(W.d_views, n_views);
+    take(W.d_jobs, n_jobs);
     A.views = W.d_views;
     A.jobs = W.d_jobs;
+    return used;
+}
+
+// The scratch for a frame of this shape. It never asks for more than the frame
+// needs: frames of many paths and frames of many records share the block, in
+// turn, without allocating, and a small frame fits wherever it fits alone. What
+// the adjoint keeps makes room where there is none.
+static cudaError_t ensure_scratch(WfScratch& W, int Q, int maxS, int iters, int n_jobs,
+                                  int n_views) {
+    maxS = std::max(maxS, 1);
+    WfScratch shape;
+    const size_t need = carve(shape, nullptr, Q, maxS, iters, n_jobs, n_views);
+    if (need > W.bytes) {
+        if (W.graph) cudaGraphExecDestroy(W.graph);
+        W.graph = nullptr;
+        if (W.mem) cudaFree(W.mem);
+        W.mem = nullptr;
+        W.bytes = 0;
+        cudaError_t e = cudaMalloc(&W.mem, need);
+        if (e == cudaErrorMemoryAllocation && W.kept) {
+            (void)cudaGetLastError();
+            cudaFree(W.kept);
+            W.kept = nullptr;
+            W.kept_bytes = 0;
+            e = cudaMalloc(&W.mem, need);
+        }
+        if (e != cudaSuccess) { W.mem = nullptr; return e; }
+        W.bytes = need;
+    }
+    carve(W, W.mem, Q, maxS, iters, n_jobs, n_views);
     return cudaSuccess;
 }
 
@@ -1453,6 +1449,7 @@ cudaError_t wavefront_render(WfScratch& W, const std::vector<SceneView>& views,
     unsigned long long key = 1469598103934665603ull;
     auto mix = [&](unsigned long long v) { key = (key ^ v) * 1099511628211ull; };
     mix((unsigned long long)n);
+    mix((unsigned long long)views.size());
     mix((unsigned long long)Q);
     mix((unsigned long long)maxS);
     mix((unsigned long long)sort_key);
@@ -1654,7 +1651,6 @@ void wavefront_release(WfScratch& W) {
     if (W.mem) cudaFree(W.mem);
     W.mem = nullptr;
     W.bytes = 0;
-    W.Q = 0;
     if (W.kept) cudaFree(W.kept);
     W.kept = nullptr;
     W.kept_bytes = 0;

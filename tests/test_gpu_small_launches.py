@@ -208,3 +208,41 @@ def test_quad_lights_are_tested_whatever_their_flag(gpu, pathtrace):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
         else:                       # FP64 sums in another order
             assert np.abs(a - b).max() <= 1e-9 * max(np.abs(b).max(), 1e-30)
+
+
+def test_scratch_holds_frames_in_turn_not_their_product(gpu):
+    """A context's scratch is the size of its largest frame: a frame of few
+    paths and many records after one of many paths and one record asks for
+    nothing, in either order, and nothing is given back and taken again
+    between them. Images stay what they were."""
+    torch = pytest.importorskip("torch")
+    from pencil_b200.renderer import GpuContext
+    few, _ = load_golden("three_spheres")
+    some, _ = load_golden("cloud2k")
+    for k in range(10):
+        some.add_light(Light.point((0.1 * k, 4.0, -3.0), (0.02, 0.02, 0.02), 0.0))
+    many, _ = load_golden("cloud2k")
+    for k in range(70):
+        many.add_light(Light.point((0.1 * k, 4.0, -3.0), (0.02, 0.02, 0.02), 0.0))
+    frames = [(few, 2048, 2048, 2), (some, 141, 142, 1), (many, 120, 90, 1)]
+    ctx = GpuContext(0)
+    sids = [ctx.upload(f[0]) for f in frames]
+    outs = [torch.empty((h, w, 3), dtype=torch.float32, device="cuda") for _, w, h, _ in frames]
+    sts = [RenderSettings(width=w, height=h, samples=n, pathtrace=True, pathtrace_bounces=3,
+                          block_size=128) for _, w, h, n in frames]
+
+    def frame(k):
+        ctx.render_device(sids[k], sts[k], outs[k].data_ptr())
+        torch.cuda.synchronize()
+        return outs[k].clone()
+
+    first = [frame(k) for k in (1, 2, 0)]       # the largest last: nothing grows from here on
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for k in (1, 0, 2, 1, 1, 0, 0, 2, 2):
+        img = frame(k)
+        assert torch.equal(img, first[(1, 2, 0).index(k)])
+        # (clones come from torch's own pool)
+        assert torch.cuda.mem_get_info()[0] >= free - (256 << 20), "scratch grew by the product"
+        assert torch.cuda.mem_get_info()[0] <= free + (256 << 20), "scratch was given back"
+    ctx.close()
