@@ -65,7 +65,8 @@ constexpr int kMaxTreeFrames = 32;     // Whitted recursion bound of the two-bra
 struct DeviceScene {
     void* arena = nullptr;             // binary nodes, leaves, vertices, materials, lights
     void* arena_wide = nullptr;        // 4-wide nodes (null when the root is a leaf)
-    size_t bytes = 0;                  // both arenas
+    void* arena_cam = nullptr;         // the same relative to the camera, where there was memory
+    size_t bytes = 0;                  // the first two arenas
     SceneView view{};
     int n_unified = 0;
     int n_leaves = 0;
@@ -273,17 +274,45 @@ cudaError_t ensure_pool(pgpu_ctx* c) {
     return cudaSuccess;
 }
 
+// Gives the scenes' camera-relative nodes back (their camera rays are traced
+// one per lane from then on); false where there are none. The stream is idle.
+bool free_camera_nodes(pgpu_ctx* c) {
+    bool any = false;
+    for (auto& s : c->scenes) {
+        DeviceScene& ds = *s.second;
+        if (!ds.arena_cam) continue;
+        cudaFreeAsync(ds.arena_cam, c->stream);
+        ds.arena_cam = nullptr;
+        ds.view.wide_cam = nullptr;
+        any = true;
+    }
+    return any;
+}
+
+// Runs alloc() (it takes device memory and returns a cudaError_t); where there
+// is none to be had, the context gives back what it only keeps to be fast, and
+// alloc() runs again: first the renders' scratch (the next render takes what
+// is left), then the camera-relative nodes of its scenes.
+template <class F>
+cudaError_t with_room(pgpu_ctx* c, F alloc) {
+    cudaError_t e = alloc();
+    for (int step = 0; step < 2 && e == cudaErrorMemoryAllocation; ++step) {
+        (void)cudaGetLastError();
+        if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return e;
+        if (step == 0) wavefront_release(*c->wf);
+        else if (!free_camera_nodes(c)) return cudaErrorMemoryAllocation;
+        if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return e;
+        if (c->pool) cudaMemPoolTrimTo(c->pool, 0);
+        e = alloc();
+    }
+    return e;
+}
+
 // Scene arena from the context's memory pool.
 cudaError_t arena_alloc(pgpu_ctx* c, size_t bytes, void** out) {
-    cudaError_t e = ensure_pool(c);
+    const cudaError_t e = ensure_pool(c);
     if (e != cudaSuccess) return e;
-    e = cudaMallocFromPoolAsync(out, bytes, c->pool, c->stream);
-    if (e != cudaErrorMemoryAllocation) return e;
-    // the renders' scratch makes room: the next render takes what is left
-    (void)cudaGetLastError();
-    if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return e;
-    wavefront_release(*c->wf);
-    return cudaMallocFromPoolAsync(out, bytes, c->pool, c->stream);
+    return with_room(c, [&] { return cudaMallocFromPoolAsync(out, bytes, c->pool, c->stream); });
 }
 
 #define PGPU_CUDA(ctx, call)                                          \
@@ -298,7 +327,9 @@ int ensure(pgpu_ctx* c, T*& ptr, size_t& cap, size_t need) {
     if (ptr) cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&ptr), std::max<size_t>(need, 256));
+    const cudaError_t e = with_room(c, [&] {
+        return cudaMalloc(reinterpret_cast<void**>(&ptr), std::max<size_t>(need, 256));
+    });
     if (e != cudaSuccess) {
         ptr = nullptr;
         return fail(c, PGPU_ERR_OUT_OF_MEMORY, "cudaMalloc(%zu): %s", need, cudaGetErrorString(e));
@@ -462,6 +493,7 @@ void pgpu_destroy(pgpu_ctx* c) {
     for (auto& kv : c->scenes) {
         cudaFreeAsync(kv.second->arena, c->stream);
         if (kv.second->arena_wide) cudaFreeAsync(kv.second->arena_wide, c->stream);
+        if (kv.second->arena_cam) cudaFreeAsync(kv.second->arena_cam, c->stream);
     }
     c->scenes.clear();
     if (c->stream) cudaStreamSynchronize(c->stream);
@@ -545,13 +577,20 @@ static cudaError_t start_tree(pgpu_ctx* c, const pgpu_scene& s, int nU, int mode
                               pgpu_bvh_node** d_table, pgpu_bvh_node* host) {
     const size_t bytes = (2 * (size_t)nU - 1) * sizeof(pgpu_bvh_node);
     *d_table = nullptr;
-    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(d_table), bytes, c->pool,
-                                            c->stream);
-    if (e != cudaSuccess) { *d_table = nullptr; return e; }
     int* depth = c->h_status + 2;
-    e = mode == PGPU_TRAVERSAL_SAH
-            ? device_sah(s, nU, *d_table, depth, c->stream, c->pool, !pencil)
-            : device_lbvh(s, nU, *d_table, depth, c->stream, c->pool);
+    cudaError_t e = with_room(c, [&] {
+        cudaError_t ae = cudaMallocFromPoolAsync(reinterpret_cast<void**>(d_table), bytes,
+                                                 c->pool, c->stream);
+        if (ae != cudaSuccess) { *d_table = nullptr; return ae; }
+        ae = mode == PGPU_TRAVERSAL_SAH
+                 ? device_sah(s, nU, *d_table, depth, c->stream, c->pool, !pencil)
+                 : device_lbvh(s, nU, *d_table, depth, c->stream, c->pool);
+        if (ae == cudaErrorMemoryAllocation) {     // (its workspace: nothing was enqueued)
+            cudaFreeAsync(*d_table, c->stream);
+            *d_table = nullptr;
+        }
+        return ae;
+    });
     if (e == cudaSuccess && host)
         e = cudaMemcpyAsync(host, *d_table, bytes, cudaMemcpyDeviceToHost, c->stream);
     return e;
@@ -967,6 +1006,7 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     auto release = [&] {
         if (ds->arena) cudaFreeAsync(ds->arena, c->stream);
         if (ds->arena_wide) cudaFreeAsync(ds->arena_wide, c->stream);
+        if (ds->arena_cam) cudaFreeAsync(ds->arena_cam, c->stream);
         cudaStreamSynchronize(c->stream);
     };
     cudaError_t e = arena_alloc(c, total, &ds->arena);
@@ -1012,16 +1052,8 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
                     wide_stack, kMaxDepth);
     }
     const size_t wide_bytes = (size_t)n_wide * kWideNodeFloat4 * 16;
-    bool relative = false;
     if (n_wide) {
-        // the nodes, and their planes relative to the camera where both fit
-        // (without, camera rays are traced one per lane)
-        if (kWideWidth == 4) {
-            e = arena_alloc(c, 2 * wide_bytes, &ds->arena_wide);
-            relative = e == cudaSuccess;
-            if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();
-        }
-        if (!relative) e = arena_alloc(c, wide_bytes, &ds->arena_wide);
+        e = arena_alloc(c, wide_bytes, &ds->arena_wide);
         if (e != cudaSuccess) {
             ds->arena_wide = nullptr;
             release();
@@ -1029,11 +1061,22 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
                         cudaGetErrorString(e));
         }
         e = cudaMemcpyAsync(ds->arena_wide, h_wide, wide_bytes, cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess && relative) {
-            camera_basis(s->camera, ds->view.cam);
-            float4* w = static_cast<float4*>(ds->arena_wide);
-            e = launch_wide_relative(w, n_wide, ds->view.cam, w + (size_t)n_wide * kWideNodeFloat4,
-                                     c->stream);
+        // the same nodes with their planes relative to the camera, where there
+        // is memory for them
+        if (e == cudaSuccess && kWideWidth == 4) {
+            e = cudaMallocFromPoolAsync(&ds->arena_cam, wide_bytes, c->pool, c->stream);
+            if (e == cudaSuccess) {
+                camera_basis(s->camera, ds->view.cam);
+                e = launch_wide_relative(static_cast<const float4*>(ds->arena_wide), n_wide,
+                                         ds->view.cam, static_cast<float4*>(ds->arena_cam),
+                                         c->stream);
+            } else {
+                ds->arena_cam = nullptr;
+                if (e == cudaErrorMemoryAllocation) {
+                    (void)cudaGetLastError();
+                    e = cudaSuccess;
+                }
+            }
         }
         if (e != cudaSuccess) {
             release();
@@ -1061,7 +1104,7 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     SceneView& v = ds->view;
     v.nodes = reinterpret_cast<const float4*>(base + off_nodes);
     v.wide = n_wide ? static_cast<const float4*>(ds->arena_wide) : nullptr;
-    v.wide_cam = relative ? v.wide + (size_t)n_wide * kWideNodeFloat4 : nullptr;
+    v.wide_cam = static_cast<const float4*>(ds->arena_cam);
     v.geo_a = reinterpret_cast<const float4*>(base + off_ga);
     v.geo_b = reinterpret_cast<const float4*>(base + off_gb);
     v.geo_c = has_tri ? reinterpret_cast<const float4*>(base + off_gc) : nullptr;
@@ -1111,6 +1154,7 @@ int32_t pgpu_free_scene(pgpu_ctx* c, int32_t id) {
     cudaStreamSynchronize(c->stream);
     cudaFreeAsync(ds->arena, c->stream);
     if (ds->arena_wide) cudaFreeAsync(ds->arena_wide, c->stream);
+    if (ds->arena_cam) cudaFreeAsync(ds->arena_cam, c->stream);
     c->scenes.erase(id);
     return PGPU_OK;
 }
@@ -1268,16 +1312,16 @@ int run_wavefront(pgpu_ctx* c, const std::vector<DeviceScene*>& scenes,
                   const std::vector<RenderCfg>& cfgs, const std::vector<float*>& outs,
                   const std::vector<float*>& m2s, bool use_graph, int* launches,
                   double* kernel_ms) {
-    std::vector<SceneView> views;
+    std::vector<DeviceScene*> distinct;
     std::vector<std::vector<DevLight>> lights;
     std::vector<int> job_view;
     std::map<const DeviceScene*, int> vidx;
     for (auto* ds : scenes) {
         auto it = vidx.find(ds);
         if (it == vidx.end()) {
-            int k = (int)views.size();
+            int k = (int)distinct.size();
             vidx[ds] = k;
-            views.push_back(ds->view);
+            distinct.push_back(ds);
             lights.push_back(ds->lights);
             job_view.push_back(k);
         } else {
@@ -1285,8 +1329,13 @@ int run_wavefront(pgpu_ctx* c, const std::vector<DeviceScene*>& scenes,
         }
     }
     *c->h_status = 0;
-    cudaError_t e = wavefront_render(*c->wf, views, lights, job_view, cfgs, outs, m2s, c->d_cnt,
-                                     c->stream, use_graph, launches, c->h_status, kernel_ms);
+    auto render = [&] {
+        std::vector<SceneView> views;
+        for (auto* ds : distinct) views.push_back(ds->view);
+        return wavefront_render(*c->wf, views, lights, job_view, cfgs, outs, m2s, c->d_cnt,
+                                c->stream, use_graph, launches, c->h_status, kernel_ms);
+    };
+    const cudaError_t e = with_room(c, render);
     if (e != cudaSuccess) return cuda_fail(c, e, "wavefront launch");
     return PGPU_OK;
 }
