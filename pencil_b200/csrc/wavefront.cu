@@ -58,9 +58,13 @@ constexpr int kSortBins = 1 << (3 * kMortonBits + 3);
 // extension rays as well for a cheaper histogram and scan).
 constexpr int kMortonBitsE = 5;
 constexpr int kSortBinsE = 1 << (3 * kMortonBitsE + 3);
-// wavefront_adjoint: paths up to which one kernel is as fast, paths per chunk.
+// wavefront_adjoint: paths up to which one kernel is as fast, the most paths
+// per chunk, and the bytes that a chunk's scratch and kept results may take
+// (the context holds them from then on): 2 GiB are 4.2M paths of one record and
+// 11 bounces, 830,000 of the 32 records and 16 bounces that are the most.
 constexpr long long kAdjOneKernel = 1 << 18;
-constexpr int kAdjChunk = 1 << 22;
+constexpr long long kAdjChunk = 1 << 22;
+constexpr long long kAdjBytes = 2LL << 30;
 
 // One render job of the path space.
 struct WfJob {
@@ -1073,6 +1077,10 @@ struct WfScratch {
     size_t kept_bytes = 0;
 };
 
+// Bytes of scratch per path in flight (carve: eight arrays of 16 bytes, two
+// queues, five lists of the sorts), beside 64 per shadow record.
+constexpr long long kPathBytes = 8 * 16 + 2 * 4 * kOctants + 5 * 4;
+
 static size_t al(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Lays out the arrays of a frame's shape from `base` in W.args, W.d_views and
@@ -1412,7 +1420,7 @@ cudaError_t wavefront_render(WfScratch& W, const std::vector<SceneView>& views,
     constexpr long long kAutoLow = 1LL << 22, kAutoHigh = 1LL << 24;
     long long cap = qcap;
     if (qcap <= 0)
-        cap = std::min(kAutoHigh, std::max(kAutoLow, (8LL << 30) / (212 + 64LL * maxS)));
+        cap = std::min(kAutoHigh, std::max(kAutoLow, (8LL << 30) / (kPathBytes + 64LL * maxS)));
     auto capacity = [&](long long want) {
         return std::max<long long>(std::min(std::max<long long>(want, max_spp), total_paths), 1);
     };
@@ -1583,10 +1591,15 @@ cudaError_t wavefront_adjoint(WfScratch& W, const SceneView& view,
     *done = false;
     const long long paths = cfg.pixels() * cfg.spp;
     const int maxS = max_shadow_records(view, lights, cfg.soft);
+    const long long chunk =
+        std::min(kAdjChunk, kAdjBytes / (kPathBytes + 64LL * maxS + 20LL * cfg.depth));
     if (!packets_for(view) || cfg.count || cfg.depth < 1 || maxS > 32 || paths <= kAdjOneKernel ||
-        cfg.spp > kAdjChunk)
+        cfg.spp > chunk)
         return cudaSuccess;
-    const long long ppc = std::min<long long>(kAdjChunk / cfg.spp, cfg.pixels());
+    // whole warps of pixels (the replay's warps sum their pixels' terms in FP32
+    // before the FP64 atomics: the same pixels share a warp in one launch)
+    long long ppc = std::min<long long>(chunk / cfg.spp, cfg.pixels());
+    if (ppc < cfg.pixels() && ppc > 32) ppc &= ~31LL;
     const int Q = (int)(ppc * cfg.spp);
     const size_t per = al((size_t)Q * 16), per_vis = al((size_t)Q * 4);
     const size_t need = (per + per_vis) * (size_t)cfg.depth;

@@ -37,6 +37,10 @@ def big_frame(ctx, sid) -> None:
 def full():
     """A context with scratch and warm kernels, in a device with 48 MiB left
     (less than any of the calls below takes)."""
+    scene = W.sphere_cloud(600_000).scene
+    other = GpuContext(0)           # (its pool keeps what the build takes)
+    nodes, depth = other.build_bvh_device(scene, "lbvh")
+    other.close()
     ctx = GpuContext(0)
     warm = W.mesh_box(3, 64, 64, 1, 2)
     for tree in (A.TRAVERSAL_LBVH, A.TRAVERSAL_SAH, A.TRAVERSAL_UPLOADED):
@@ -45,8 +49,6 @@ def full():
         ctx.render(sid, warm.settings)
     for method in ("sah", "lbvh"):
         ctx.build_bvh_device(warm.scene, method)
-    scene = W.sphere_cloud(600_000).scene
-    nodes, depth = ctx.build_bvh_device(scene, "lbvh")
     big_frame(ctx, sid)
     held = fill(48 << 20)
     yield ctx, scene, nodes, sid, warm
@@ -100,4 +102,31 @@ def test_scenes_give_their_camera_nodes(gpu):
     torch.cuda.empty_cache()
     assert np.array_equal(ctx.render(a, st), want1)
     assert np.array_equal(ctx.render(b, st), want2)
+    ctx.close()
+
+
+def test_adjoint_keeps_at_most_two_gigabytes(gpu):
+    """The most records and bounces that the queued adjoint takes, in a frame
+    of more paths than one chunk of them: the same gradients in chunks."""
+    import dataclasses
+    from conftest import load_golden
+    from pencil_b200.scene import Light
+    scene, _ = load_golden("three_spheres")
+    scene.lights = [Light.point((k - 3.5, 4.0, -3.0), (0.1, 0.1, 0.1), 0.4) for k in range(8)]
+    st = RenderSettings(width=1024, height=1030, samples=2, max_depth=16, pathtrace=True,
+                        pathtrace_bounces=16, soft_shadow_samples=4)
+    dl = np.random.default_rng(4).normal(size=(st.height, st.width, 3)).astype(np.float32)
+    ctx = GpuContext(0)
+    sid = ctx.upload(scene)
+    nm, nl = scene.n_materials, len(scene.lights)
+    b = ctx.adjoint(sid, dataclasses.replace(st, count_rays=True), dl, nm, nl, want_image=True)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    a = ctx.adjoint(sid, st, dl, nm, nl, want_image=True)
+    torch.cuda.synchronize()
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert 1 << 30 < taken <= (2 << 30) + (64 << 20)
+    assert np.array_equal(a[3].view(np.uint32), b[3].view(np.uint32))
+    for x, y in zip(a[:3], b[:3]):
+        assert np.abs(x - y).max() <= 1e-9 * max(np.abs(y).max(), 1e-30)
     ctx.close()
