@@ -40,8 +40,9 @@ struct RayCount {
 // the same for every sample of a vertex, and three normalizations (square
 // roots and divisions): a loop over samples takes them once (Whitted room of 63
 // primitives, 1.2M paths, four samples: 1.28 -> 1.20 ms; 64x64 tiles 4-5%
-// less), but in the wavefront's shading kernel (kDiscOnce), where the axes'
-// registers spill and path-traced frames pay for it (0.3%).
+// less), but in the wavefront's shading kernel (kDiscOnce) and the adjoint,
+// where the axes' registers spill and path-traced frames and gradients pay for
+// it (0.3%, 3%).
 struct LightDisc {
     V3 t1, t2;
 };
