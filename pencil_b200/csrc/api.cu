@@ -78,6 +78,8 @@ struct DeviceScene {
     bool has_glass = false;            // a dielectric material (two-branch glass needs it)
     bool has_reflective = false;       // a material that continues a Whitted path
     bool has_long_kinds = false;       // cubes, cylinders or cones
+    bool has_walls = false;            // see has_walls()
+    bool mostly_triangles = false;     // three quarters of the primitives or more
     std::vector<DevLight> lights;
     std::vector<int> quad_mats;        // material ids of quad-light emitters
     DevMaterial* d_mats = nullptr;
@@ -569,6 +571,31 @@ int32_t pgpu_build_bvh(const pgpu_scene* s, pgpu_bvh_node* out_nodes, int32_t* o
 }
 
 }  // extern "C"
+
+// Whether a leaf's box has at least a quarter of the scene box's surface: a
+// wall, a ground plane, a floor. Rays of such a scene hit something at nearly
+// every bounce, where those of a cloud or a lone object mostly leave. (A box
+// that large lies in boxes at least as large: the search goes down only those.)
+static bool has_walls(const pgpu_bvh_node* nodes, int n_nodes) {
+    auto area = [&](int k) {
+        const float* a = nodes[k].bmin;
+        const float* b = nodes[k].bmax;
+        const double x = (double)b[0] - a[0], y = (double)b[1] - a[1], z = (double)b[2] - a[2];
+        return x * y + y * z + z * x;
+    };
+    if (n_nodes < 2) return false;
+    const double least = 0.25 * area(0);
+    std::vector<int> todo{0};
+    while (!todo.empty()) {
+        const int k = todo.back();
+        todo.pop_back();
+        if (!(area(k) >= least)) continue;
+        if (nodes[k].left < 0) return true;
+        todo.push_back(nodes[k].left);
+        todo.push_back(nodes[k].right);
+    }
+    return false;
+}
 
 // Enqueues a device build of mode `mode` (PGPU_TRAVERSAL_LBVH, _SAH; `pencil`:
 // Pencil's SAH tree) into a table from the context's pool (*d_table, to be
@@ -1094,6 +1121,13 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
         const int t = s->prims[k].type;
         return t == PGPU_PRIM_CUBE || t == PGPU_PRIM_CYLINDER || t == PGPU_PRIM_CONE;
     }) >= 0;
+    std::atomic<long long> tri_prims{0};
+    parallel_for(s->n_prims, [&](int b, int e2) {
+        long long k = 0;
+        for (int i = b; i < e2; ++i) k += s->prims[i].type == PGPU_PRIM_TRIANGLE ? 1 : 0;
+        tri_prims += k;
+    });
+    const long long n_tri = s->n_mesh_triangles + tri_prims.load();
     e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         release();
@@ -1135,6 +1169,8 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     ds->has_glass = has_glass;
     ds->has_reflective = has_reflective;
     ds->has_long_kinds = has_long_kinds;
+    ds->has_walls = has_walls(nodes, n_nodes);
+    ds->mostly_triangles = n_tri * 4 >= 3LL * nU;
     ds->lights = std::move(lights);
     ds->quad_mats = std::move(quad_mats);
     ds->d_mats = reinterpret_cast<DevMaterial*>(base + off_mt);
@@ -1341,37 +1377,77 @@ int run_wavefront(pgpu_ctx* c, const std::vector<DeviceScene*>& scenes,
 }
 
 // Whether a frame of the wavefront engine runs as one kernel, a thread per
-// path (mk_render, which makes the same image bit for bit), instead of the
-// queued kernels. Queues pay three kernels a bounce, each as long as its
+// path (mk_render, which makes the image of the queues with camera rays one per
+// lane bit for bit, and of camera packets but for cones: their sides lie
+// outside the box that the reference gives them, so that the walk's order
+// decides which rays find them), instead of the queued kernels. Queues pay three kernels a bounce, each as long as its
 // longest ray; one kernel pays once, but its warps run their paths' parts in
 // turn, which costs more the more rays there are and the more they diverge.
-// So the line is drawn by the rays of a first vertex, and by what makes them
-// diverge: the depth of the tree and the kinds of primitives. Queued / one
-// kernel, ms, by paths:
-//   path tracing, one light, up to 1024 leaves: 4 leaves 0.33 / 0.19 (528k),
-//     0.45 / 0.46 (1.1M); 300 leaves 0.30 / 0.12 (528k); three lights, 62
-//     triangles 0.59 / 0.40 (128k), 0.91 / 1.13 (528k)
-//   more leaves: 5,000 spheres 0.42 / 0.26 (128k), 0.55 / 0.56 (528k); 100,000
-//     spheres 1.32 / 0.99 (64k), 1.47 / 1.49 (128k); 5,000 triangles 0.82 /
-//     0.81 (128k); 328,000 triangles 1.51 / 1.05 (128k)
-//   cubes, cylinders or cones, three lights: 63 leaves 1.00 / 0.83 (64k), 1.10
-//     / 1.49 (128k); 253 leaves 1.59 / 1.40 (24k), 1.92 / 2.67 (64k)
-//   Whitted mode, where only glass and metal continue: 63 leaves 1.08 / 0.43
-//     (230k), 10.5 / 7.4 (14.7M); 328,000 triangles without glass or metal
-//     14.8 / 10.6 (14.7M); 303 leaves 2.6 / 1.6 (230k), 4.0 / 4.7 (1.2M);
-//     20,000 spheres 0.61 / 0.50 (230k), 1.06 / 1.63 (1.2M)
+// Measured on 48 scenes of 4 to 328,000 primitives, depths 2 to 16, 8,000 to
+// 8 million paths (one kernel's time / the queues'):
+//
+// Path tracing. Queues cost by the bounce, so the number of paths at which the
+// two meet grows with the depth (measured from 4 to 16). What it is per bounce
+// depends on whether paths end early (has_walls), on how far a ray walks (the
+// number of primitives, less so among triangles) and on what its lanes do at a
+// leaf (cubes, cylinders, cones):
+//   open, up to 1,024 primitives or triangles: 1,000 spheres 0.88 at 524k paths
+//     and depth 4, 0.60 at 16; 82,000 triangles 0.93, 0.66
+//   open, more: 5,000 spheres 0.91 at 131k and 4; 20,000 spheres 0.63 at 32k,
+//     1.27 at 131k; 100,000 spheres 0.72 and 1.57
+//   walls (by the rays of a vertex): 338 triangles in a box 0.81 at 32k and 4,
+//     1.21 at 131k, at 16 0.87 and 1.28 at 524k; 1,018 spheres 0.81, 1.26,
+//     0.76, 1.31; three lights, 250 spheres and triangles 0.80, 1.68, 0.88,
+//     1.84; 82,000 triangles 0.73, 1.04, 0.72, 1.10
+//   cubes, cylinders, cones, three lights: 23 primitives 0.86 at 32k and 4, 1.70
+//     at 131k; 63: 0.99, 2.06; 253: 0.76 at 8k, 1.18 at 32k; 903: 0.81, 1.35
+//   up to 8 primitives: 0.81 at 262k and 4, 1.14 at 524k; six lights 1.01
+//
+// Whitted mode, where only glass and metal continue: the lights' samples, which
+// the queues write and read as records, are most of the work.
+//   matte: triangles 0.45-0.89 at every size, with four more soft lights 0.5; 300
+//     spheres 1.04 at 8.4M paths; 20,000 spheres 0.73 at 131k, 1.27 at 524k
+//   glass or metal: up to 64 primitives, and up to 256 without cubes, cylinders
+//     and cones, 0.6-1.0 at 8.4M; 1,003 spheres and triangles 0.87 at 524k, 1.31
+//     at 2.1M; 20,000 spheres 0.73 at 131k, 1.35 at 524k; 100,000 0.94, 1.68
+//   with cubes, cylinders, cones (more samples of a pixel make neighbouring
+//     paths alike): 1 sample and 6 records a vertex, 63 primitives 1.01 at 2.1M,
+//     123: 0.83 at 524k, 1.21 at 2.1M, 253: 1.04 at 524k, 1.58 at 2.1M, but 0.66
+//     and 1.01 with 18 records, 1.37 and 2.08 with 3; 16 samples 0.75, 0.92,
+//     1.14 at 2.1M, at 14.7M 63 primitives 0.82, 103: 0.90; 4 samples, 63: 0.96
+//     at 8.4M, 153: 0.87 at 1M, 1.16 at 4.1M
 // Frames that count, profile or set a launch parameter keep the queues.
 static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
     if (c.count || c.profile || !c.packets || c.queue_capacity || c.sort_key || c.refill ||
         c.block || std::getenv("PGPU_INJECT_SHADOW_RECORDS"))
         return false;
     const long long paths = c.pixels() * c.spp;
-    if (c.mode == PGPU_MODE_WHITTED)
-        return ds.n_leaves <= 256 || !ds.has_reflective || paths <= (1 << 18);
-    long long rays = 1;                 // of a path-traced vertex
+    const int n = ds.n_leaves;
+    if (c.mode == PGPU_MODE_WHITTED) {
+        if (!ds.has_reflective) return n <= 1024 || ds.mostly_triangles || paths <= 1 << 18;
+        if (n > 256) return paths <= (n <= 65536 || ds.mostly_triangles ? 1 << 18 : 1 << 17);
+        if (!ds.has_long_kinds || n <= 32) return true;
+        long long records = 0;              // of a vertex
+        for (const DevLight& l : ds.lights)
+            if (l.kind != PGPU_LIGHT_QUAD) records += l.radius > 0.0f ? c.soft : 1;
+        if (n <= 128 && c.spp >= (n <= 64 ? 4 : 16)) return true;
+        const long long each = n <= 64 ? 1 << 18 : n <= 128 ? 1 << 17 : 3 << 15;
+        return paths <= each * std::max(records, 1LL) * (c.spp >= 16 ? 8 : c.spp >= 4 ? 2 : 1);
+    }
+    long long rays = 1;                     // of a path-traced vertex
     for (const DevLight& l : ds.lights) rays += l.is_emissive ? 0 : 1;
-    const long long most = ds.has_long_kinds ? 1 << 17 : ds.n_leaves <= 1024 ? 1 << 20 : 1 << 18;
-    return paths * rays <= most;
+    long long per;                          // 1024 paths per bounce
+    if (n <= 8) {
+        per = 96;
+        rays = 1;
+    }
+    else if (ds.has_long_kinds) per = n <= 32 ? 40 : n <= 64 ? 32 : n <= 256 ? 22 : 15;
+    else if (ds.has_walls) per = n <= 64 || n > 32768 ? 48 : 28;
+    else {
+        per = n <= 1024 || ds.mostly_triangles ? 128 : n <= 8192 ? 32 : n <= 32768 ? 16 : 12;
+        rays = 1;
+    }
+    return paths * rays <= per * 1024 * std::min(std::max(c.depth, 4), 16);
 }
 
 // pgpu_render and pgpu_render_window: the image, or the window `win` of it.
