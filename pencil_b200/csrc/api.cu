@@ -17,6 +17,8 @@
 #include <thread>
 #include <vector>
 
+#include <sys/mman.h>
+
 #include "host_internal.h"
 
 namespace pgpu {
@@ -150,6 +152,8 @@ struct pgpu_ctx {
     int* h_status = nullptr;          // pinned
     unsigned char* h_stage = nullptr; // pinned staging of scene uploads
     size_t stage_cap = 0;
+    void* stage_map = nullptr;        // the mapping it lies in (null: cudaMallocHost's)
+    size_t stage_map_bytes = 0;
     unsigned char* d_adj = nullptr;   // adjoint inputs and gradient sums
     size_t adj_cap = 0;
     uint8_t* d_rgb8 = nullptr;        // tonemap output staging
@@ -340,18 +344,59 @@ int ensure(pgpu_ctx* c, T*& ptr, size_t& cap, size_t need) {
     return PGPU_OK;
 }
 
-// Pinned host memory of at least `need` bytes (contents lost when it grows).
-int ensure_pinned(pgpu_ctx* c, unsigned char*& p, size_t& cap, size_t need) {
-    if (cap >= need) return PGPU_OK;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
-    cap = 0;
-    if (cudaMallocHost(reinterpret_cast<void**>(&p), need) != cudaSuccess) {
+void free_stage(pgpu_ctx* c) {
+    if (c->stage_map) {
+        cudaHostUnregister(c->h_stage);
+        munmap(c->stage_map, c->stage_map_bytes);
+    } else if (c->h_stage) {
+        cudaFreeHost(c->h_stage);
+    }
+    c->h_stage = nullptr;
+    c->stage_cap = 0;
+    c->stage_map = nullptr;
+}
+
+// Pinned staging of at least `need` bytes (contents lost when it grows). A
+// context's first upload waited for its pages above all: cudaMallocHost takes
+// 17.8 ms for 27 MB, all of it faults of 4 KB pages. So the staging lies in 2 MB
+// pages where the system has them, touched by the host threads before it is
+// registered (first upload of a context: 82k triangles with a tree of their own
+// 26.4 -> 7.4 ms, 50,000 spheres 19.8 -> 4.0; median of 24 contexts).
+int ensure_stage(pgpu_ctx* c, size_t need) {
+    if (c->stage_cap >= need) return PGPU_OK;
+    free_stage(c);
+    constexpr size_t kHuge = 2 << 20, kPage = 4096;
+    if (need >= kHuge) {
+        const size_t bytes = (need + kHuge - 1) & ~(kHuge - 1);
+        void* m = mmap(nullptr, bytes + kHuge, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS,
+                       -1, 0);
+        if (m != MAP_FAILED) {
+            unsigned char* p = reinterpret_cast<unsigned char*>(
+                (reinterpret_cast<uintptr_t>(m) + kHuge - 1) & ~(uintptr_t)(kHuge - 1));
+            madvise(p, bytes, MADV_HUGEPAGE);
+            // (a child of a fork must not make the parent's pages copies)
+            madvise(p, bytes, MADV_DONTFORK);
+            host_run((int)(bytes / kHuge), [&](int t) {
+                volatile unsigned char* q = p + t * kHuge;
+                for (size_t b = 0; b < kHuge; b += kPage) q[b] = 0;
+            });
+            if (cudaHostRegister(p, bytes, cudaHostRegisterDefault) == cudaSuccess) {
+                c->h_stage = p;
+                c->stage_cap = bytes;
+                c->stage_map = m;
+                c->stage_map_bytes = bytes + kHuge;
+                return PGPU_OK;
+            }
+            (void)cudaGetLastError();
+            munmap(m, bytes + kHuge);
+        }
+    }
+    if (cudaMallocHost(reinterpret_cast<void**>(&c->h_stage), need) != cudaSuccess) {
         (void)cudaGetLastError();
-        p = nullptr;
+        c->h_stage = nullptr;
         return fail(c, PGPU_ERR_OUT_OF_MEMORY, "pinned staging of %zu bytes", need);
     }
-    cap = need;
+    c->stage_cap = need;
     return PGPU_OK;
 }
 
@@ -509,7 +554,7 @@ void pgpu_destroy(pgpu_ctx* c) {
     cudaFree(c->d_tone);
     wavefront_delete(c->wf);
     if (c->h_status) cudaFreeHost(c->h_status);
-    if (c->h_stage) cudaFreeHost(c->h_stage);
+    free_stage(c);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
     if (c->ev_tree) cudaEventDestroy(c->ev_tree);
@@ -882,7 +927,7 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     const size_t wide_cap = align256((size_t)n_int * kWideNodeFloat4 * 16);
     const bool own_tree = c->traversal != PGPU_TRAVERSAL_UPLOADED && nU >= 2;
     const size_t tree_cap = own_tree ? (2 * (size_t)nU - 1) * sizeof(pgpu_bvh_node) : 0;
-    int rc = ensure_pinned(c, c->h_stage, c->stage_cap, total + wide_cap + tree_cap);
+    int rc = ensure_stage(c, total + wide_cap + tree_cap);
     if (rc) return rc;
     // A traversal tree of its own needs only the primitives: the device builds
     // it while the host checks and converts the uploaded one (82k triangles:

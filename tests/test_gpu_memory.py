@@ -130,3 +130,20 @@ def test_adjoint_keeps_at_most_two_gigabytes(gpu):
     for x, y in zip(a[:3], b[:3]):
         assert np.abs(x - y).max() <= 1e-9 * max(np.abs(y).max(), 1e-30)
     ctx.close()
+
+
+@pytest.mark.parametrize("tree", [A.TRAVERSAL_UPLOADED, A.TRAVERSAL_LBVH])
+def test_staging_grows_with_the_scenes(tree):
+    """Uploads of one context whose staging is below 2 MB, above, below again
+    (what is there is kept) and far above: each scene renders as it does in a
+    context of its own."""
+    ctx = GpuContext(0)
+    ctx.set_traversal_tree(tree)
+    for n in (300, 9_000, 300, 60_000, 9_000):
+        w = W.sphere_cloud(n, 160, 90, 1, 3)
+        own = GpuContext(0)
+        own.set_traversal_tree(tree)
+        a, b = (c.render(c.upload(w.scene), w.settings) for c in (ctx, own))
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), n
+        own.close()
+    ctx.close()
