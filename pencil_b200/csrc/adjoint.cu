@@ -318,8 +318,11 @@ struct Replay {
 // latency (per gradient: 16.45 ms; 17.49 at 80 registers, 16.70 at 64).
 constexpr int kAdjMinBlocks = 7;
 // A launch of one wave at four blocks per SM waits for its longest paths, not
-// for issue slots, and gets 128 registers (12,288 paths 0.203 -> 0.191 ms; 76,800,
-// just beyond the line, would gain 0.53 -> 0.47, 120,000 lose 0.67 -> 0.71).
+// for issue slots, and gets 128 registers (12,288 paths 0.203 -> 0.191 ms). The
+// line is the wave: 76,800 threads, eight blocks more, would still gain 7-15%
+// (30 to 1,000 spheres, depth 3 to 6), but 81,920 would lose 4-15% on frames of one
+// sample and gain or lose 7% on those of nine, 98,304 lose 8-16%, 144,300 lose or
+// gain 4%.
 constexpr int kAdjSmallBlocks = 4;
 constexpr long long kAdjSmallThreads = 148LL * kAdjSmallBlocks * kAdjBlock;
 

@@ -1384,7 +1384,11 @@ int make_cfg(pgpu_ctx* c, const DeviceScene* ds, const pgpu_render_params* p, Re
     cfg.block = p->block_size;
     cfg.win[0] = cfg.win[1] = cfg.win[2] = cfg.win[3] = 0;
     cfg.worker = false;
-    (void)ds;
+    cfg.records = 0;
+    for (const DevLight& l : ds->lights) {
+        if (l.is_emissive || (l.kind == PGPU_LIGHT_QUAD && cfg.mode == PGPU_MODE_WHITTED)) continue;
+        cfg.records += cfg.mode == PGPU_MODE_WHITTED && l.radius > 0.0f ? cfg.soft : 1;
+    }
     return PGPU_OK;
 }
 

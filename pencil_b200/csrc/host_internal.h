@@ -57,6 +57,7 @@ struct RenderCfg {
     int block;        // wavefront threads per block (0: the default)
     int win[4];       // window x, y, w, h of the image (w = 0: the whole image)
     bool worker;      // the distributed worker's jitter (render_tile)
+    long long records;  // shadow rays that a vertex's lights ask for, at most
     long long pixels() const { return win[2] > 0 ? (long long)win[2] * win[3] : (long long)W * H; }
 };
 

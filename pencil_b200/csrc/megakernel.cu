@@ -24,17 +24,19 @@ constexpr int kMkMinBlocks = 8;
 // lanes per pixel in the reference-exact mode.
 cudaError_t launch_mk_small(const SceneView& S, const PathParams& P, int G, long long threads,
                             float* out, float* m2, cudaStream_t st, bool* done);
-cudaError_t launch_mk_team(const SceneView& S, const PathParams& P, bool wide, long long pixels,
-                           float* out, float* m2, cudaStream_t st, bool* done);
+cudaError_t launch_mk_team(const SceneView& S, const PathParams& P, bool wide, long long records,
+                           long long pixels, float* out, float* m2, cudaStream_t st, bool* done);
 
 template <bool COUNT, bool TREE, bool PIXEL_SEQ, bool WIDE>
-static cudaError_t launch_mk(const SceneView& S, const PathParams& P, int G, float* out,
-                             float* m2, unsigned long long* counters, cudaStream_t st) {
+static cudaError_t launch_mk(const SceneView& S, const PathParams& P, int G, long long records,
+                             float* out, float* m2, unsigned long long* counters,
+                             cudaStream_t st) {
     const long long threads =
         (P.tile_w > 0 ? (long long)P.tile_w * P.tile_h : (long long)P.W * P.H) * G;
     if constexpr (!COUNT && ((TREE && PIXEL_SEQ) || (!TREE && !PIXEL_SEQ && WIDE))) {
         bool done = false;
-        const cudaError_t e = TREE ? launch_mk_team(S, P, WIDE, threads, out, m2, st, &done)
+        const cudaError_t e = TREE ? launch_mk_team(S, P, WIDE, records, threads, out, m2, st,
+                                                    &done)
                                    : launch_mk_small(S, P, G, threads, out, m2, st, &done);
         if (done || e != cudaSuccess) return e;
     }
@@ -58,8 +60,8 @@ cudaError_t launch_megakernel(const SceneView& S, const RenderCfg& c, float* out
     const bool wide = !c.binary_tree;
 #define PGPU_MK_CASE(CNT, TR, SQ)                                                \
     if (c.count == CNT && tree == TR && seq == SQ)                               \
-        return wide ? launch_mk<CNT, TR, SQ, true>(S, P, G, out, m2, counters, st) \
-                    : launch_mk<CNT, TR, SQ, false>(S, P, G, out, m2, counters, st);
+        return wide ? launch_mk<CNT, TR, SQ, true>(S, P, G, c.records, out, m2, counters, st) \
+                    : launch_mk<CNT, TR, SQ, false>(S, P, G, c.records, out, m2, counters, st);
     PGPU_MK_CASE(false, false, false)
     PGPU_MK_CASE(false, false, true)
     PGPU_MK_CASE(false, true, false)

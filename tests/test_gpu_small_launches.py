@@ -53,6 +53,29 @@ def test_more_shadow_rays_than_lanes(gpu, soft, binary_tree):
     gpu.free(sid)
 
 
+# the last size of each group and the first of the next, by the shadow rays of a
+# vertex (hard lights; 0: a light that is not tested)
+@pytest.mark.parametrize("pathtrace,lights,pixels", [
+    (True, 0, 64), (True, 1, 4736), (True, 2, 4736), (True, 2, 7104), (True, 3, 4736),
+    (True, 6, 7104), (False, 0, 64), (False, 1, 9472), (False, 1, 37888), (False, 2, 9472),
+    (False, 2, 75776), (False, 4, 37888), (False, 6, 18944), (False, 6, 75776)])
+def test_lane_groups_by_shadow_rays(gpu, pathtrace, lights, pixels):
+    scene, _ = load_golden("prims_mix")
+    scene.lights[:] = [Light.point((0.7 * k - 2, 4, -3), (0.6, 0.5, 0.4), 0.0)
+                       for k in range(max(lights, 1))]
+    if lights == 0:
+        scene.lights[0] = dataclasses.replace(scene.lights[0], is_emissive=True)
+    sid = gpu.upload(scene)
+    for n in (pixels, pixels + 1):
+        st = RenderSettings(width=n, height=1, samples=1, max_depth=3, pathtrace=pathtrace,
+                            pathtrace_bounces=3, engine=A.ENGINE_MEGAKERNEL,
+                            rng=A.RNG_PIXEL_SEQUENTIAL, glass=A.GLASS_BOTH_BRANCHES)
+        a = gpu.render(sid, st)
+        b = gpu.render(sid, dataclasses.replace(st, count_rays=True))
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    gpu.free(sid)
+
+
 # frames that run as one kernel unless a launch parameter asks for the queues
 @pytest.mark.parametrize("name", ["three_spheres", "prims_mix", "cloud2k", "mesh_small", "shapes"])
 @pytest.mark.parametrize("pathtrace", [False, True])
