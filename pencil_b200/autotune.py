@@ -19,7 +19,10 @@ workload (image size, samples, scene, light count) and the GPU:
 
 `autotune` times candidates with short device-resident renders (CUDA events
 on the render stream, a warm-up render first) by coordinate search: capacity
-first, then the refill threshold, the sort key and the block size. Results
+first, then the refill threshold, the sort key and the block size. A single
+frame is timed once more with none of them set: any of them keeps a frame on
+the queued kernels, and a small frame may be faster as the one kernel that the
+renderer then picks (all four 0 in the result). Results
 are cached in a JSON file keyed by the workload's shape, so a renderer pays
 the search once.
 """
@@ -133,7 +136,17 @@ def autotune(ctx: GpuContext, sids: list[int], settings: list[RenderSettings], s
                   t["block_size"] == b_best)
     best = {"queue_capacity": q_best, "refill_below": r_best, "sort_key": s_best,
             "block_size": b_best, "ms": best_ms}
-    apply(q_best, r_best, s_best, b_best)
+    # with none set (frames that would fit a chunk: larger ones run on the
+    # queues but for matte scenes and small rooms in Whitted mode)
+    if len(sids) == 1 and total_paths <= fit[-1]:
+        apply(0, 0, 0, 0)
+        ms = _time_device(ctx, render, reps)
+        if log:
+            log(f"autotune untuned: {ms:.2f} ms")
+        if ms < best_ms:
+            best = {"queue_capacity": 0, "refill_below": 0, "sort_key": 0, "block_size": 0,
+                    "ms": ms}
+    apply(best["queue_capacity"], best["refill_below"], best["sort_key"], best["block_size"])
     if use_cache and key:
         cache[key] = best
         try:

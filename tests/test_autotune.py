@@ -119,3 +119,32 @@ def test_signature_follows_the_workload_shape():
     t = FakeScene()
     t.n_unified = 1001
     assert T.signature(s, a) != T.signature(t, a)
+
+
+@pytest.mark.parametrize("untuned_ms,frames,taken", [(5.0, 1, True), (10.5, 1, False),
+                                                     (5.0, 2, False)])
+def test_a_small_frame_is_tried_without_launch_parameters(tuner, monkeypatch, untuned_ms, frames,
+                                                          taken):
+    """Any launch parameter keeps a frame on the queues; one that is faster as
+    one kernel is left without them (a batch never runs as one kernel)."""
+    ctx, _ = tuner
+    settings = [RenderSettings(width=64, height=64, samples=1, pathtrace=True,
+                               pathtrace_bounces=4) for _ in range(frames)]
+
+    def cost(c, render, reps):
+        render()
+        st = settings[0]
+        if not (st.queue_capacity or st.refill_below or st.sort_key or st.block_size):
+            return untuned_ms
+        return 10.0 + (st.refill_below - 16) ** 2
+    monkeypatch.setattr(T, "_time_device", cost)
+    out = T.autotune(ctx, list(range(frames)), settings, scene=FakeScene(), reps=1)
+    knobs = ("queue_capacity", "refill_below", "sort_key", "block_size")
+    assert (out["ms"] == untuned_ms) == taken
+    for st in settings:
+        assert [getattr(st, k) for k in knobs] == [out[k] for k in knobs]
+        assert (not any(getattr(st, k) for k in knobs)) == taken
+    fresh = [RenderSettings(width=64, height=64, samples=1, pathtrace=True, pathtrace_bounces=4)
+             for _ in range(frames)]
+    again = T.autotune(ctx, list(range(frames)), fresh, scene=FakeScene(), reps=1)
+    assert again["cached"] and [getattr(fresh[0], k) for k in knobs] == [out[k] for k in knobs]
