@@ -61,13 +61,13 @@ const GammaThresholds& thresholds() {
 
 }  // namespace
 
-// Exactly, the byte of a clamped value is found in two steps: the
-// value's exponent and top 7 mantissa bits pick a cell whose lower end has
-// `base` thresholds at or below it, and no cell holds a second threshold (a
-// cell is 1/128 of its octave; the closest thresholds of the top octave lie
-// 1.5 cells apart, those of lower octaves further; the host checks it), so
-// one comparison with t[base + 1] finishes the count. Values below 2^-20 lie
-// below t[1] = (0.5 / 255)^2.2.
+// Exactly, the byte of a clamped value is found in two steps: the value's
+// exponent and top 7 mantissa bits pick a cell whose lower end has `base`
+// thresholds at or below it, and the count goes on from there. (A cell is 1/128
+// of its octave, so it holds one threshold at most: the closest of the top
+// octave lie 1.5 cells apart, those of lower octaves further. The count does not
+// rely on it.) Values below 2^-20, which is below t[1] = (0.5 / 255)^2.2, have
+// no cell.
 constexpr int kCellShift = 23 - 7;
 constexpr uint32_t kCellFirst = 0x35800000u;             // 2^-20
 constexpr int kCells = (int)((0x3f800000u - kCellFirst) >> kCellShift) + 1;   // up to 1.0
@@ -103,10 +103,11 @@ __device__ __noinline__ uint32_t tone_byte(float x, const ToneTable* __restrict_
         x = x / (1.0f + x);
     }
     x = (x < 0.0f) ? 0.0f : (x > 1.0f) ? 1.0f : x;     // clampf
-    // below the first cell (and NaN): no threshold is at or below the value
-    if (!(x >= __uint_as_float(kCellFirst))) return 0;
-    const uint32_t k = __ldg(&table->base[(__float_as_uint(x) - kCellFirst) >> kCellShift]);
-    return k + (__ldg(&table->t[k + 1]) <= x ? 1u : 0u);
+    uint32_t k = 0;                    // (NaN: no threshold is at or below it)
+    if (x >= __uint_as_float(kCellFirst))
+        k = __ldg(&table->base[(__float_as_uint(x) - kCellFirst) >> kCellShift]);
+    while (__ldg(&table->t[k + 1]) <= x) ++k;
+    return k;
 }
 
 // The byte as 255 y^(1/2.2) rounded, from the hardware's approximate
