@@ -1499,6 +1499,64 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
     return paths * rays <= per * 1024 * std::min(std::max(c.depth, 4), 16);
 }
 
+// Whether a gradient is traced as it is replayed, in one kernel, instead of
+// replaying what the queued kernels found (wavefront_adjoint). Queues pay by the
+// bounce and by the path's kept state; one kernel's warps run their paths' parts
+// in turn, so that it loses by what makes paths of a warp unlike (walls that
+// keep paths going for different numbers of bounces, lights of several kinds,
+// cubes, cylinders and cones, long walks in large trees), and by the lanes left
+// idle where a pixel's lanes divide its samples unevenly (9 samples of 8
+// lanes). Measured on 44 scenes, depths 1 to 16, 262k to 8.4M paths (one
+// kernel's time / the queues'):
+//
+// Path tracing
+//   open: 300 and 2,000 spheres 0.15-1.06, with six more lights 0.25-0.75; 5,000 at
+//     1.0M paths and depths to 8 0.79-1.40; 20,000 at 360k and depth 4 1.13, at
+//     705k and 16 0.92; 100,000 1.04-2.7
+//   walls, one light, even samples: 30 spheres 0.52-0.98; 120 0.65-1.00 up to 705k,
+//     0.76-1.19 beyond; 1,000 0.75-1.02 at 360k, 1.22-1.43 from 1.4M at depths 4
+//     and 8, but 0.89-1.08 at every size at depth 2; 338 to 5,000 triangles
+//     0.59-1.04, 20,000 0.70-1.15, 82,000 0.76-0.98 at 360k, 1.05-1.30 beyond 1M;
+//     depth 1 all 0.43-1.00
+//   uneven: 30 spheres 0.56-1.05 up to 1.0M, 0.75-1.17 beyond; 120 0.72-0.98 at 275k,
+//     1.06-1.30 at 1.0M; 1,000 0.82-1.24 at 275k, 1.24-1.80 beyond 1M
+//   walls, more lights: 30 spheres and three lights 0.94-1.30 at 360k, 1.20-2.4
+//     beyond; with cubes, cylinders and cones 0.8-4.2
+//   three spheres: 0.22-0.81, with three lights 0.30-1.06, with eight 0.37-1.24
+// Whitted mode: even samples 0.13-0.97 but for 20,000 spheres (0.65-0.99 at
+//   360k, 1.0-1.45 beyond 1M); uneven, with walls, 0.77-1.42 at depths 2 and 4
+//   (1.0M), 0.26-1.36 at 8 and 16
+// Large frames that set a launch parameter keep the queues, as renders do.
+static bool one_kernel_adjoint(const DeviceScene& ds, const RenderCfg& c) {
+    const long long paths = c.pixels() * c.spp;
+    const int n = ds.n_leaves, depth = c.depth;
+    if (paths <= 1 << 18) return true;
+    if (c.queue_capacity || c.sort_key || c.refill || c.block || !c.packets) return false;
+    const bool whitted = c.mode == PGPU_MODE_WHITTED;
+    const double small = (whitted ? 2e9 : 1e9) * depth;     // paths x leaves
+    if (!ds.has_walls) return n <= 2500 || (double)paths * n <= small;
+    if (n <= 8)
+        return c.records <= (whitted ? 4 : 3) || depth <= 2 || paths <= (long long)depth << 17;
+    int lanes = 1;
+    while (lanes * 2 <= std::min(c.spp, 32)) lanes *= 2;
+    const bool even = (c.spp + lanes - 1) / lanes * lanes * 4 <= c.spp * 5;
+    if (whitted) {
+        if (n > 256 && ds.has_long_kinds) return false;
+        if (n > 4096 && !ds.mostly_triangles) return (double)paths * n <= small;
+        return even || paths <= (long long)depth << 17;
+    }
+    if (ds.has_long_kinds || c.records > 1) return false;
+    if (depth <= 1) return n <= 32768 || ds.mostly_triangles;
+    const bool easy = n <= 50 || (ds.mostly_triangles && n <= 32768);
+    if (even && (easy || depth <= 2)) return true;
+    if (easy && depth <= 2) return true;
+    long long most;                                         // 1024 paths
+    if (even) most = n <= 144 ? 640 : 384;
+    else if (easy) most = 700;
+    else most = depth <= 2 ? (n <= 144 ? 700 : 256) : n <= 144 ? 320 : 200;
+    return paths <= most * 1024 * (depth >= 12 ? 2 : 1);
+}
+
 // pgpu_render and pgpu_render_window: the image, or the window `win` of it.
 static int32_t render_impl(pgpu_ctx* c, int32_t id, const pgpu_render_params* p,
                            const int32_t* win, float* out_rgb, float* out_m2, pgpu_stats* stats) {
@@ -1756,8 +1814,9 @@ int32_t pgpu_adjoint(pgpu_ctx* c, int32_t id, const pgpu_render_params* p, const
     const AdjointOut ao{d_dl, d_g, d_g + 3 * nm, d_g + 6 * nm, out_rgb ? d_img : nullptr, c->d_cnt};
     int launches = 1;
     bool done = false;
-    cudaError_t e = wavefront_adjoint(*c->wf, ds->view, ds->lights, cfg, ao, c->stream, &launches,
-                                      &done);
+    cudaError_t e = cudaSuccess;
+    if (!one_kernel_adjoint(*ds, cfg))
+        e = wavefront_adjoint(*c->wf, ds->view, ds->lights, cfg, ao, c->stream, &launches, &done);
     if (e == cudaSuccess && !done) e = launch_adjoint(ds->view, cfg, ao, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "adjoint launch");
     PGPU_CUDA(c, cudaEventRecord(c->ev1, c->stream));

@@ -58,11 +58,9 @@ constexpr int kSortBins = 1 << (3 * kMortonBits + 3);
 // extension rays as well for a cheaper histogram and scan).
 constexpr int kMortonBitsE = 5;
 constexpr int kSortBinsE = 1 << (3 * kMortonBitsE + 3);
-// wavefront_adjoint: paths up to which one kernel is as fast, the most paths
-// per chunk, and the bytes that a chunk's scratch and kept results may take
-// (the context holds them from then on): 2 GiB are 4.2M paths of one record and
+// wavefront_adjoint: the most paths per chunk, and the bytes that a chunk's
+// scratch and kept results may take (the context holds them from then on): 2 GiB are 4.2M paths of one record and
 // 11 bounces, 830,000 of the 32 records and 16 bounces that are the most.
-constexpr long long kAdjOneKernel = 1 << 18;
 constexpr long long kAdjChunk = 1 << 22;
 constexpr long long kAdjBytes = 2LL << 30;
 
@@ -1578,23 +1576,18 @@ cudaError_t launch_adjoint_found(const SceneView& S, const RenderCfg& c, const A
 // forward once, every bounce's hits and shadow results kept (20 bytes per path
 // and bounce), and the replay that differentiates them traces nothing. The
 // kernel that traces as it replays keeps 5 of a warp's 32 lanes busy, as the
-// megakernel does. Per gradient of the box of 1,000 spheres, one kernel /
-// this: 17.3 / 11.6 ms at 4.2M paths, 4.64 / 3.43 at 1.05M, 3.67 / 2.27 at 590k,
-// 1.32 / 1.32 at 262k (100 spheres 0.61 / 0.79), 0.66 / 0.89 at 120k; so frames
-// of up to kAdjOneKernel paths keep the one kernel, and so do counting calls
-// and scenes whose vertices have more records than a word has bits. Sets
-// *done where the pass was made. The replay's arithmetic and the order of its
-// sums are the same.
+// megakernel does. (Which frames are faster this way: one_kernel_adjoint in
+// api.cu.) Counting calls and scenes whose vertices have more records than a
+// word has bits are left to that kernel. Sets *done where the pass was made. The
+// replay's arithmetic and the order of its sums are the same.
 cudaError_t wavefront_adjoint(WfScratch& W, const SceneView& view,
                               const std::vector<DevLight>& lights, const RenderCfg& cfg,
                               const AdjointOut& o, cudaStream_t st, int* launches, bool* done) {
     *done = false;
-    const long long paths = cfg.pixels() * cfg.spp;
     const int maxS = max_shadow_records(view, lights, cfg.soft);
     const long long chunk =
         std::min(kAdjChunk, kAdjBytes / (kPathBytes + 64LL * maxS + 20LL * cfg.depth));
-    if (!packets_for(view) || cfg.count || cfg.depth < 1 || maxS > 32 || paths <= kAdjOneKernel ||
-        cfg.spp > chunk)
+    if (!packets_for(view) || cfg.count || cfg.depth < 1 || maxS > 32 || cfg.spp > chunk)
         return cudaSuccess;
     // whole warps of pixels (the replay's warps sum their pixels' terms in FP32
     // before the FP64 atomics: the same pixels share a warp in one launch)

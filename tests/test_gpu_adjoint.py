@@ -14,7 +14,7 @@ import pytest
 from oracle import oracle as O
 from pencil_b200 import _abi as A
 from pencil_b200 import workloads as W
-from pencil_b200.renderer import RenderSettings
+from pencil_b200.renderer import RenderSettings, RenderStats
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -203,4 +203,80 @@ def test_adjoint_from_the_queued_kernels_is_the_traced_one(gpu, name, size, dept
     # and the context's renders are what they were
     img = gpu.render(sid, st)
     assert np.array_equal(img, gpu.render(sid, dataclasses.replace(st, block_size=128)))
+    gpu.free(sid)
+
+
+@pytest.mark.parametrize("name,size,depth,pathtrace", [
+    ("prims_mix", (171, 171, 3), 6, True), ("prims_mix", (171, 171, 3), 4, False),
+    ("three_spheres", (257, 256, 2), 16, True), ("adjoint_small", (256, 257, 2), 5, True),
+    ("cloud2k", (345, 331, 7), 2, True), ("cornell_box", (300, 225, 8), 1, True)])
+def test_adjoint_on_the_queues_of_any_scene(gpu, name, size, depth, pathtrace):
+    """A launch parameter has any large gradient take its hits and visibility
+    from the queued kernels, also those that are traced in one kernel without."""
+    import dataclasses
+    from conftest import load_golden
+    w, h, n = size
+    scene, _ = load_golden(name)
+    if name == "adjoint_small":
+        scene = W.adjoint_box(60, w, h, n, depth, seed=9)[0].scene
+    st = RenderSettings(width=w, height=h, samples=n, max_depth=depth, pathtrace=pathtrace,
+                        pathtrace_bounces=depth, seed=11)
+    sid = gpu.upload(scene)
+    dl = np.random.default_rng(2).normal(size=(h, w, 3)).astype(np.float32)
+    nm, nl = scene.n_materials, len(scene.lights)
+    stats = RenderStats()
+    out = []
+    for kw in (dict(block_size=128), dict(sort_key=1), dict(count_rays=True)):
+        out.append(gpu.adjoint(sid, dataclasses.replace(st, **kw), dl, nm, nl, stats=stats,
+                               want_image=True))
+        assert (stats.kernel_launches > 1) == (len(out) < 3)
+    for a in out[:2]:
+        assert np.array_equal(a[3].view(np.uint32), out[2][3].view(np.uint32))
+        for x, y in zip(a[:3], out[2][:3]):
+            assert np.abs(x - y).max() <= 1e-9 * max(np.abs(y).max(), 1e-30)
+    gpu.free(sid)
+
+
+# scene, path tracing, lights added, depth, samples, the largest width x height of
+# one kernel (0: any)
+LINES = [("box60", True, 0, 4, 1, (1024, 640)), ("box60", True, 0, 12, 3, (256, 284)),
+         ("box60", True, 1, 4, 1, (512, 512)), ("box300", True, 0, 4, 2, (384, 256)),
+         ("box300", True, 0, 2, 2, None), ("box300", True, 0, 4, 3, (172, 169)),
+         ("box30", True, 0, 6, 3, (280, 284)), ("mesh5k", True, 0, 6, 2, None),
+         ("cloud5k", True, 0, 2, 1, (800, 500)), ("cloud5k", False, 0, 2, 1, (1000, 800)),
+         ("three_spheres", True, 4, 3, 1, (768, 512)), ("box60", False, 1, 3, 3, (256, 170)),
+         ("box60", False, 1, 3, 2, None), ("cloud300", True, 3, 4, 2, None)]
+
+
+@pytest.mark.parametrize("name,pathtrace,lights,depth,samples,size", LINES)
+def test_which_gradients_run_as_one_kernel(gpu, name, pathtrace, lights, depth, samples, size):
+    """Both sides of the line that the scene's kind, depth and samples draw:
+    the image of the counting call, which always runs as one kernel."""
+    import dataclasses
+    from conftest import load_golden
+    from pencil_b200.scene import Light
+    if name == "three_spheres":
+        scene, _ = load_golden(name)
+    elif name == "mesh5k":
+        scene = W.mesh_box(4, 64, 64).scene
+    elif name.startswith("box"):
+        scene = W.adjoint_box(int(name[3:]), 64, 64, 1, 4, seed=9)[0].scene
+    else:
+        scene = W.sphere_cloud({"300": 300, "5k": 5000}[name[5:]]).scene
+    for k in range(lights):
+        scene.add_light(Light.point((k - 2, 4, -3), (0.1, 0.2, 0.1), 0.0))
+    sid = gpu.upload(scene)
+    nm, nl = scene.n_materials, len(scene.lights)
+    for extra in (0, 1):
+        w, h = (size[0], size[1] + extra) if size else (700 + extra, 701)
+        st = RenderSettings(width=w, height=h, samples=samples, max_depth=depth,
+                            pathtrace=pathtrace, pathtrace_bounces=depth)
+        dl = np.random.default_rng(2).normal(size=(h, w, 3)).astype(np.float32)
+        stats = RenderStats()
+        a = gpu.adjoint(sid, st, dl, nm, nl, stats=stats, want_image=True)
+        assert (stats.kernel_launches == 1) == (size is None or extra == 0)
+        b = gpu.adjoint(sid, dataclasses.replace(st, count_rays=True), dl, nm, nl, want_image=True)
+        assert np.array_equal(a[3].view(np.uint32), b[3].view(np.uint32))
+        for x, y in zip(a[:3], b[:3]):
+            assert np.abs(x - y).max() <= 1e-9 * max(np.abs(y).max(), 1e-30)
     gpu.free(sid)
