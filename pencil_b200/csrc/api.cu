@@ -1425,6 +1425,14 @@ int run_wavefront(pgpu_ctx* c, const std::vector<DeviceScene*>& scenes,
     return PGPU_OK;
 }
 
+// Whether a pixel's samples keep its lanes of one kernel busy alike: 1, 4, 16 or
+// 64 do, 9 (two turns of 8 lanes), 25, 36 or 49 keep a fifth to a half idle.
+static bool even_samples(int spp) {
+    int lanes = 1;
+    while (lanes * 2 <= std::min(spp, 32)) lanes *= 2;
+    return (spp + lanes - 1) / lanes * lanes * 4 <= spp * 5;
+}
+
 // Whether a frame of the wavefront engine runs as one kernel, a thread per
 // path (mk_render, which makes the image of the queues with camera rays one per
 // lane bit for bit, and of camera packets but for cones: their sides lie
@@ -1465,6 +1473,15 @@ int run_wavefront(pgpu_ctx* c, const std::vector<DeviceScene*>& scenes,
 //     and 1.01 with 18 records, 1.37 and 2.08 with 3; 16 samples 0.75, 0.92,
 //     1.14 at 2.1M, at 14.7M 63 primitives 0.82, 103: 0.90; 4 samples, 63: 0.96
 //     at 8.4M, 153: 0.87 at 1M, 1.16 at 4.1M
+//
+// Uneven samples (even_samples; above, all are even) cost one kernel more the
+// larger the frame. 9 samples, Whitted: three spheres 0.98 at 2.1M paths and
+// depth 4; rooms of 23 and 63 primitives 0.98 and 1.03 at 1.0M, 0.95 and 1.00 at 2.1M
+// and depth 10, 103: 0.90 at 263k, 1.32 at 1.0M, 253: 1.09, 1.53; matte: 312
+// spheres 0.71 at 66k, 1.08 at 263k, 338 triangles 0.98 at 1.0M, 5,138: 0.73 at
+// 66k, 1.10 at 263k, 82,000: 0.69, 1.20; 20,000 spheres of every kind 0.72, 1.36.
+// Path tracing: walls 1.22-1.42 at 66k and depth 4 (even 0.88-0.96), 0.93-1.09 at
+// 16k; three spheres 1.16 at 263k (even 0.84); open scenes as above.
 // Frames that count, profile or set a launch parameter keep the queues.
 static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
     if (c.count || c.profile || !c.packets || c.queue_capacity || c.sort_key || c.refill ||
@@ -1472,7 +1489,14 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
         return false;
     const long long paths = c.pixels() * c.spp;
     const int n = ds.n_leaves;
+    const bool even = even_samples(c.spp);
     if (c.mode == PGPU_MODE_WHITTED) {
+        if (!even) {
+            const long long k = n <= 8 ? 512                // 1024 paths per bounce
+                : n <= (ds.mostly_triangles ? 512 : ds.has_reflective ? 64 : 8) ? 256
+                : n <= 128 && ds.has_reflective ? 100 : n <= 8192 ? 64 : 32;
+            if (paths > k * 1024 * std::min(c.depth, 16)) return false;
+        }
         if (!ds.has_reflective) return n <= 1024 || ds.mostly_triangles || paths <= 1 << 18;
         if (n > 256) return paths <= (n <= 65536 || ds.mostly_triangles ? 1 << 18 : 1 << 17);
         if (!ds.has_long_kinds || n <= 32) return true;
@@ -1487,7 +1511,7 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
     for (const DevLight& l : ds.lights) rays += l.is_emissive ? 0 : 1;
     long long per;                          // 1024 paths per bounce
     if (n <= 8) {
-        per = 96;
+        per = even ? 96 : 48;
         rays = 1;
     }
     else if (ds.has_long_kinds) per = n <= 32 ? 40 : n <= 64 ? 32 : n <= 256 ? 22 : 15;
@@ -1496,6 +1520,7 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
         per = n <= 1024 || ds.mostly_triangles ? 128 : n <= 8192 ? 32 : n <= 32768 ? 16 : 12;
         rays = 1;
     }
+    if (!even && n > 8 && (ds.has_long_kinds || ds.has_walls)) rays *= 4;
     return paths * rays <= per * 1024 * std::min(std::max(c.depth, 4), 16);
 }
 
@@ -1537,9 +1562,7 @@ static bool one_kernel_adjoint(const DeviceScene& ds, const RenderCfg& c) {
     if (!ds.has_walls) return n <= 2500 || (double)paths * n <= small;
     if (n <= 8)
         return c.records <= (whitted ? 4 : 3) || depth <= 2 || paths <= (long long)depth << 17;
-    int lanes = 1;
-    while (lanes * 2 <= std::min(c.spp, 32)) lanes *= 2;
-    const bool even = (c.spp + lanes - 1) / lanes * lanes * 4 <= c.spp * 5;
+    const bool even = even_samples(c.spp);
     if (whitted) {
         if (n > 256 && ds.has_long_kinds) return false;
         if (n > 4096 && !ds.mostly_triangles) return (double)paths * n <= small;

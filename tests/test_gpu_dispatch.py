@@ -122,3 +122,14 @@ def test_frames_of_one_kernel_at_any_size(gpu, name):
     b = gpu.render(sid, queued(name, st))
     assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
     gpu.free(sid)
+
+
+# samples that a pixel's lanes share unevenly (9 of 8 lanes, 25 of 16)
+@pytest.mark.parametrize("name,pathtrace,depth,samples,size", [
+    ("spheres", True, 4, 3, (182, 120)), ("spheres", False, 3, 3, (512, 341)),
+    ("box338", True, 4, 3, (64, 24)), ("box338", False, 3, 3, (256, 341)),
+    ("room123", False, 2, 3, (256, 88)), ("room20", False, 2, 5, (256, 81)),
+    ("matte20000", False, 4, 3, (128, 113)), ("lone5120", False, 4, 3, (128, 227)),
+    ("cloud300", True, 4, 3, (256, 227))])
+def test_lines_of_uneven_samples(gpu, name, pathtrace, depth, samples, size):
+    test_both_sides_of_each_line(gpu, name, pathtrace, depth, samples, size)
