@@ -350,6 +350,9 @@ def run_ours(args) -> None:
     ctx.render(sid, st, stats=prof)
     ctx.render(sid, st, stats=prof)
     st.profile_kernels = False
+    # (the rays of the counting render: closest hits and a shadow ray per light
+    # sample, as the reference traces; the timed frame leaves out the shadow rays
+    # whose term is zero, so it traces fewer than this)
     rays = cnt.extension_rays + cnt.shadow_rays
     mrays = rays * world / (ms_wf * 1e-3) / 1e6
 
@@ -493,6 +496,8 @@ def run_ours(args) -> None:
                                       "NCCL all-reduce of the image per step" if world > 1
                                       else "1 GPU"},
             "mrays_per_s": mrays,
+            "mrays_note": "rays of the estimator (a shadow ray per light sample); those whose "
+                          "term is zero are counted but not traced in the timed frame",
             "rays_per_step": rays,
             # Pencil's own count (RenderStats::rays_traced: one per trace /
             # trace_path call), for comparison with the reference's figures

@@ -132,7 +132,8 @@ typedef struct pgpu_light {
                                the light travels; quad: corner              */
     float   intensity[3];   /* point/directional: intensity; quad: radiance */
     float   radius;         /* point: soft-shadow disc radius (0 = hard)    */
-    int32_t is_emissive;    /* point: skip the shadow test                  */
+    int32_t is_emissive;    /* point, directional: skip the shadow test (a
+                               quad is tested whatever it says)             */
     float   edge_u[3];      /* quad: first edge from the corner             */
     float   edge_v[3];      /* quad: second edge from the corner            */
     int32_t material;       /* quad: material of the emitter surface        */
@@ -176,7 +177,13 @@ enum pgpu_mode {
 };
 
 enum pgpu_engine {
-    PGPU_ENGINE_WAVEFRONT  = 0, /* persistent generate/extend/shade/shadow    */
+    /* Persistent camera/extend/shade/shadow kernels over queues of paths. A
+     * frame that is too small for queues to pay, and sets none of
+     * queue_capacity, refill_below, sort_key, block_size, PGPU_FLAG_NO_PACKETS,
+     * ray counting and profiling, runs as one kernel, a thread per path: the
+     * same image, but where the sides of a cone, which lie outside the box that
+     * Pencil gives it, make the order of a walk decide whether a ray finds it. */
+    PGPU_ENGINE_WAVEFRONT  = 0,
     PGPU_ENGINE_MEGAKERNEL = 1  /* one thread per path, all bounces in one
                                    kernel                                    */
 };
@@ -205,12 +212,12 @@ enum pgpu_flags {
     PGPU_FLAG_DEVICE_OUTPUT = 1,  /* out_rgb / out_m2 are device pointers   */
     PGPU_FLAG_COUNT_RAYS    = 2,  /* fill the ray counters in pgpu_stats    */
     PGPU_FLAG_COUNT_NODES   = 4,  /* also count node visits / prim tests    */
-    PGPU_FLAG_NO_GRAPH      = 8,  /* wavefront: launch kernels one by one
-                                     instead of replaying a CUDA graph       */
+    PGPU_FLAG_NO_GRAPH      = 8,  /* wavefront: launch the queues' kernels one
+                                     by one instead of replaying a CUDA graph */
     PGPU_FLAG_PROFILE_KERNELS = 16, /* time each kernel class (implies
                                      NO_GRAPH); see pgpu_stats.kernel_ms     */
-    PGPU_FLAG_NO_PACKETS    = 32, /* wavefront: trace camera rays one per lane
-                                     instead of as warp packets              */
+    PGPU_FLAG_NO_PACKETS    = 32, /* wavefront: queues with camera rays traced
+                                     one per lane instead of as warp packets */
     PGPU_FLAG_MIS           = 64, /* path tracing with trace_path_mis's light
                                      weights (RenderSettings::mis,
                                      src/renderer.hpp:55, 1205-1346)         */
@@ -234,17 +241,21 @@ typedef struct pgpu_render_params {
     uint32_t seed;              /* salt mixed into the counter RNG (0: none) */
     int32_t  sample_offset;     /* first sample index (progressive renders)  */
     int32_t  flags;             /* enum pgpu_flags                           */
-    int32_t  queue_capacity;    /* wavefront paths in flight, 0..2^28 (0:
+    /* Wavefront launch parameters; any that is set keeps a frame (and a
+     * gradient of more than 2^18 paths) on the queues. */
+    int32_t  queue_capacity;    /* paths in flight, 0..2^28 (0: automatic, up to
+                                   2^24 as far as 8 GiB of scratch hold them,
+                                   at least 2^22)                            */
+    int32_t  refill_below;      /* a warp takes new rays once at most this many
+                                   of its 32 lanes are still traversing (0:
                                    automatic)                                */
-    int32_t  refill_below;      /* wavefront: a warp takes new rays once at
-                                   most this many of its 32 lanes are still
-                                   traversing (0: automatic)                 */
-    int32_t  sort_key;          /* wavefront ray order: 0 queue order, 1 binned
+    int32_t  sort_key;          /* ray order: 0 queue order, 1 binned
                                    by direction octant, 2 shadow work sorted
                                    by origin (Morton code) and octant, 3 also
                                    the extension rays of bounces >= 1        */
-    int32_t  block_size;        /* wavefront threads per block: 64, 128 or 256
-                                   (0: 128; pgpu_render_noalloc always 128)  */
+    int32_t  block_size;        /* threads per block of the queues' kernels: 64,
+                                   128 or 256 (0: 128; pgpu_render_noalloc
+                                   always 128)                               */
 } pgpu_render_params;
 
 typedef struct pgpu_stats {
@@ -265,7 +276,8 @@ typedef struct pgpu_stats {
      * extend, shade, shadow, accumulate, megakernel), from CUDA events
      * around every launch (kernels are then launched one by one). */
     double   kernel_ms[6];
-    int32_t  kernel_launches;  /* kernels launched by the call               */
+    int32_t  kernel_launches;  /* kernels launched by the call (a frame that
+                                  replays a CUDA graph: 1)                   */
     int32_t  reserved;
 } pgpu_stats;
 
@@ -300,7 +312,7 @@ int32_t pgpu_set_timeout(pgpu_ctx* ctx, int32_t ms);
  * equal distance as BVHNode::hit does (src/bvh.hpp:31-37), so hit
  * distances are the same and images agree but where rounding at a box face
  * makes the order of the walk matter. The binary tree the upload keeps
- * (PGPU_FLAG_BINARY_TREE, the adjoint) is the uploaded one in both modes.
+ * (PGPU_FLAG_BINARY_TREE, the ray queries) is the uploaded one in all modes.
  *   PGPU_TRAVERSAL_UPLOADED (0, default): the uploaded tree (Pencil's SAH
  *       tree), collapsed to wide nodes.
  *   PGPU_TRAVERSAL_LBVH (1): a linear BVH over the uploaded leaves, built on
@@ -353,8 +365,9 @@ int32_t pgpu_build_bvh_device(pgpu_ctx* ctx, const pgpu_scene* scene,
 
 /* Pencil's own SAH tree (BVH::build, src/bvh.hpp:74-192: 12 buckets along
  * the longest axis, cost 1 + (nL SA_L + nR SA_R) / SA_P, median split for
- * <= 4 primitives and when no bucket boundary separates) built on the GPU,
- * one tree level at a time, in the same table format. Splits are those of
+ * <= 4 primitives and when no bucket boundary separates) built on the GPU in
+ * the same table format: nodes of more than 512 primitives one tree level at
+ * a time, each subtree below them by one block. Splits are those of
  * the host build; the sides of a split keep their primitives in a stable
  * order where Pencil's std::partition does not, so trees agree node for node
  * unless two primitives tie in a median split's centroid key. out_nodes
@@ -371,8 +384,11 @@ int32_t pgpu_free_scene(pgpu_ctx* ctx, int32_t scene_id);
 /* Sizes of an uploaded scene. No counterpart in the reference (Pencil keeps
  * its scene on the host): it reports what pgpu_upload_scene built. */
 typedef struct pgpu_scene_info {
-    int64_t device_bytes;      /* bytes of the scene's device arena, all copied
-                                  from pinned host memory by the upload      */
+    /* Bytes of the scene's device arena, all copied from pinned host memory by
+     * the upload. A second copy of its wide nodes (128 bytes each), relative to
+     * the camera and made on the device, is not among them: it is given back
+     * where memory runs short. */
+    int64_t device_bytes;
     int32_t n_leaves;          /* primitives (one per BVH leaf)              */
     int32_t n_interior;        /* interior nodes of the binary tree          */
     int32_t n_wide;            /* wide nodes collapsed from it               */
@@ -385,7 +401,13 @@ int32_t pgpu_get_scene_info(pgpu_ctx* ctx, int32_t scene_id, pgpu_scene_info* ou
 /* Render one image: out_rgb gets width*height*3 floats, row-major, row 0 at
  * the top, each pixel the mean of its n*n samples (the layout of
  * Renderer::render's std::vector<Color>). out_m2 (optional) gets the
- * per-pixel mean of the squared sample radiance. */
+ * per-pixel mean of the squared sample radiance.
+ *
+ * A context keeps the queues' scratch, one block as large as its largest frame
+ * so far needed (212 bytes per path in flight and 64 per shadow record of it;
+ * queue_capacity bounds it). The context's own uploads, tree builds and output
+ * buffers take it back where memory runs short; other users of the GPU get it
+ * with pgpu_destroy. */
 int32_t pgpu_render(pgpu_ctx* ctx, int32_t scene_id,
                     const pgpu_render_params* params,
                     float* out_rgb, float* out_m2, pgpu_stats* stats);
@@ -425,7 +447,9 @@ int32_t pgpu_primary_hits(pgpu_ctx* ctx, int32_t scene_id, const float* uv,
  * accumulates dL/d(albedo) and dL/d(emission) per material (3 doubles per
  * material each) and dL/d(intensity) per light (3 doubles per light).
  * Gradient buffers are overwritten. Optional out_rgb receives the forward
- * image of the same samples. */
+ * image of the same samples. Large frames keep what a pass of the queued
+ * kernels found, with its scratch at most 2 GiB, which the context holds like
+ * a render's. */
 int32_t pgpu_adjoint(pgpu_ctx* ctx, int32_t scene_id,
                      const pgpu_render_params* params, const float* dl_dimage,
                      double* d_albedo, double* d_emission, double* d_light,
