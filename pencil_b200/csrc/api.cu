@@ -380,7 +380,8 @@ int ensure_stage(pgpu_ctx* c, size_t need) {
                 volatile unsigned char* q = p + t * kHuge;
                 for (size_t b = 0; b < kHuge; b += kPage) q[b] = 0;
             });
-            if (cudaHostRegister(p, bytes, cudaHostRegisterDefault) == cudaSuccess) {
+            // (portable, as cudaMallocHost's: the caller's current device may be another)
+            if (cudaHostRegister(p, bytes, cudaHostRegisterPortable) == cudaSuccess) {
                 c->h_stage = p;
                 c->stage_cap = bytes;
                 c->stage_map = m;
@@ -1434,12 +1435,13 @@ static bool even_samples(int spp) {
 }
 
 // Whether a frame of the wavefront engine runs as one kernel, a thread per
-// path (mk_render, which makes the image of the queues with camera rays one per
-// lane bit for bit, and of camera packets but for cones: their sides lie
-// outside the box that the reference gives them, so that the walk's order
-// decides which rays find them), instead of the queued kernels. Queues pay three kernels a bounce, each as long as its
-// longest ray; one kernel pays once, but its warps run their paths' parts in
-// turn, which costs more the more rays there are and the more they diverge.
+// path, instead of the queued kernels. mk_render makes the image of queues with
+// camera rays one per lane bit for bit, and of camera packets but for cones:
+// their sides lie outside the box that the reference gives them, so that the
+// walk's order decides which rays find them. Queues pay three kernels a bounce,
+// each as long as its longest ray; one kernel pays once, but its warps run
+// their paths' parts in turn, which costs more the more rays there are and the
+// more they diverge.
 // Measured on 48 scenes of 4 to 328,000 primitives, depths 2 to 16, 8,000 to
 // 8 million paths (one kernel's time / the queues'):
 //
