@@ -794,7 +794,7 @@ sah_local(const SahTask* local, const int* n_local, int* perm, const DBox* boxes
     constexpr int kWarps = kSahBlock / 32;
     constexpr int kTasks = kSahLocal / 5 + 1;
     __shared__ DBox s_box[kSahLocal];
-    __shared__ int s_prim[kSahLocal], s_perm[kSahLocal], s_tmp[kSahLocal];
+    __shared__ int s_prim[kSahLocal], s_perm[kSahLocal], s_tmp[kSahLocal], s_key[kSahLocal];
     __shared__ SahTask s_task[2][kTasks];
     __shared__ int s_n[2];
     __shared__ SahBin s_bin[kWarps][kSahBuckets];
@@ -904,12 +904,14 @@ sah_local(const SahTask* local, const int* n_local, int* perm, const DBox* boxes
                     int lo[2][3], hi[2][3];
                     for (int h = 0; h < 2; ++h)
                         for (int a = 0; a < 3; ++a) { lo[h][a] = ord(1e30f); hi[h][a] = ord(-1e30f); }
+                    for (int i = lane; i < count; i += 32)
+                        s_key[off + i] = ord(sah_key2(s_box[s_perm[off + i]], axis) + 0.0f);
+                    __syncwarp();
                     for (int i = lane; i < count; i += 32) {
-                        const int q = s_perm[off + i];
-                        const int key = ord(sah_key2(s_box[q], axis) + 0.0f);
+                        const int q = s_perm[off + i], key = s_key[off + i];
                         int rank = 0;
                         for (int j = 0; j < count; ++j) {
-                            const int kj = ord(sah_key2(s_box[s_perm[off + j]], axis) + 0.0f);
+                            const int kj = s_key[off + j];
                             rank += (kj < key || (kj == key && j < i)) ? 1 : 0;
                         }
                         s_tmp[off + rank] = q;
