@@ -1287,6 +1287,8 @@ int32_t pgpu_tonemap(pgpu_ctx* c, const float* hdr, int32_t n_pixels, int32_t to
     if (!c->d_tone) {
         size_t bytes = 0;
         const void* table = tone_table_host(&bytes);
+        if (!table)
+            return fail(c, PGPU_ERR_UNSUPPORTED, "gamma thresholds of this host's powf are too close");
         int rc = ensure(c, c->d_tone, c->tone_cap, bytes);
         if (rc) return rc;
         PGPU_CUDA(c, cudaMemcpy(c->d_tone, table, bytes, cudaMemcpyHostToDevice));

@@ -37,6 +37,15 @@ def gamma_thresholds() -> np.ndarray:
     return lo.view(np.float32)
 
 
+def test_no_cell_of_the_byte_table_holds_two_thresholds():
+    """What the device's table relies on (and the library checks): cells of 1/128
+    octave from 2^-20 on, one threshold in each at most."""
+    t = gamma_thresholds()
+    assert t[0] >= np.float32(2.0 ** -20)
+    cells = (t.view(np.uint32) - np.float32(2.0 ** -20).view(np.uint32)) >> 16
+    assert len(np.unique(cells)) == 255
+
+
 @pytest.mark.gpu
 def test_device_tonemap_equals_host_bytes(gpu):
     t = gamma_thresholds()
