@@ -180,9 +180,8 @@ enum pgpu_engine {
     /* Persistent camera/extend/shade/shadow kernels over queues of paths. A
      * frame that is too small for queues to pay, and sets none of
      * queue_capacity, refill_below, sort_key, block_size, PGPU_FLAG_NO_PACKETS,
-     * ray counting and profiling, runs as one kernel, a thread per path: the
-     * same image, but where the sides of a cone, which lie outside the box that
-     * Pencil gives it, make the order of a walk decide whether a ray finds it. */
+     * ray counting and profiling, runs as one kernel, a thread per path (of a
+     * scene with cones after a kernel for its camera rays): the same image. */
     PGPU_ENGINE_WAVEFRONT  = 0,
     PGPU_ENGINE_MEGAKERNEL = 1  /* one thread per path, all bounces in one
                                    kernel                                    */
@@ -217,7 +216,11 @@ enum pgpu_flags {
     PGPU_FLAG_PROFILE_KERNELS = 16, /* time each kernel class (implies
                                      NO_GRAPH); see pgpu_stats.kernel_ms     */
     PGPU_FLAG_NO_PACKETS    = 32, /* wavefront: queues with camera rays traced
-                                     one per lane instead of as warp packets */
+                                     one per lane instead of as warp packets
+                                     (the same image but for cones, whose
+                                     sides lie outside the boxes Pencil gives
+                                     them: the order of the walk decides which
+                                     rays find them)                         */
     PGPU_FLAG_MIS           = 64, /* path tracing with trace_path_mis's light
                                      weights (RenderSettings::mis,
                                      src/renderer.hpp:55, 1205-1346)         */

@@ -20,7 +20,8 @@ BUILD = HERE / "_build"
 LIB = HERE / "libpencil_gpu.so"
 INCLUDE = HERE.parent / "include"
 
-CU_SOURCES = ["api.cu", "megakernel.cu", "megakernel_small.cu", "wavefront.cu", "queries.cu", "adjoint.cu",
+CU_SOURCES = ["api.cu", "megakernel.cu", "megakernel_small.cu",
+              "megakernel_found.cu", "megakernel_found_small.cu", "wavefront.cu", "queries.cu", "adjoint.cu",
               "tonemap.cu", "bvh_device.cu"]
 CXX_SOURCES = ["bvh_build.cpp", "bvh_wide.cpp", "host_pool.cpp"]
 HEADERS = ["device_common.cuh", "path.cuh", "megakernel.cuh", "scene_layout.h", "host_internal.h"]

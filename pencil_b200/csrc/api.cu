@@ -23,8 +23,9 @@
 
 namespace pgpu {
 
-cudaError_t launch_megakernel(const SceneView& S, const RenderCfg& c, float* out, float* m2,
-                              unsigned long long* counters, cudaStream_t st);
+cudaError_t launch_megakernel(const SceneView& S, const RenderCfg& c, const float4* found,
+                              float* out, float* m2, unsigned long long* counters,
+                              cudaStream_t st);
 cudaError_t launch_wide_relative(const float4* wide, int n_wide, const float* origin, float4* out,
                                  cudaStream_t st);
 cudaError_t launch_query(const SceneView& S, bool camera, const float* in, int n, int* prim,
@@ -51,6 +52,8 @@ cudaError_t launch_adjoint(const SceneView& S, const RenderCfg& c, const Adjoint
 cudaError_t wavefront_adjoint(WfScratch& W, const SceneView& view,
                               const std::vector<DevLight>& lights, const RenderCfg& cfg,
                               const AdjointOut& o, cudaStream_t st, int* launches, bool* done);
+cudaError_t wavefront_camera_hits(WfScratch& W, const SceneView& view, const RenderCfg& cfg,
+                                  cudaStream_t st, const float4** hits);
 int adjoint_max_depth();
 int adjoint_max_lights();
 cudaError_t launch_tonemap(const float* d_hdr, long long n_pixels, int mode, float exposure,
@@ -80,6 +83,7 @@ struct DeviceScene {
     bool has_glass = false;            // a dielectric material (two-branch glass needs it)
     bool has_reflective = false;       // a material that continues a Whitted path
     bool has_long_kinds = false;       // cubes, cylinders or cones
+    bool has_cones = false;
     bool has_walls = false;            // see has_walls()
     bool mostly_triangles = false;     // three quarters of the primitives or more
     std::vector<DevLight> lights;
@@ -1167,6 +1171,9 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
         const int t = s->prims[k].type;
         return t == PGPU_PRIM_CUBE || t == PGPU_PRIM_CYLINDER || t == PGPU_PRIM_CONE;
     }) >= 0;
+    const bool has_cones = has_long_kinds && first_bad(s->n_prims, [&](int k) {
+        return s->prims[k].type == PGPU_PRIM_CONE;
+    }) >= 0;
     std::atomic<long long> tri_prims{0};
     parallel_for(s->n_prims, [&](int b, int e2) {
         long long k = 0;
@@ -1215,6 +1222,7 @@ int32_t pgpu_upload_scene(pgpu_ctx* c, const pgpu_scene* s, int32_t* out_id) {
     ds->has_glass = has_glass;
     ds->has_reflective = has_reflective;
     ds->has_long_kinds = has_long_kinds;
+    ds->has_cones = has_cones;
     ds->has_walls = has_walls(nodes, n_nodes);
     ds->mostly_triangles = n_tri * 4 >= 3LL * nU;
     ds->lights = std::move(lights);
@@ -1437,10 +1445,13 @@ static bool even_samples(int spp) {
 }
 
 // Whether a frame of the wavefront engine runs as one kernel, a thread per
-// path, instead of the queued kernels. mk_render makes the image of queues with
-// camera rays one per lane bit for bit, and of camera packets but for cones:
-// their sides lie outside the box that the reference gives them, so that the
-// walk's order decides which rays find them. Queues pay three kernels a bounce,
+// path, instead of the queued kernels: the same image bit for bit. (The sides of
+// cones lie outside the box that the reference gives them, so that the walk's
+// order decides which rays find them, and packets take another than lanes of
+// their own. Frames of scenes with cones therefore have their camera rays
+// traced as the queues trace them, first, where one chunk of the queues would
+// hold them; in 4 of 110 rooms that showed, in 2 to 22 pixels, where the packets
+// agree with the reference's order.) Queues pay three kernels a bounce,
 // each as long as its longest ray; one kernel pays once, but its warps run
 // their paths' parts in turn, which costs more the more rays there are and the
 // more they diverge.
@@ -1494,6 +1505,7 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
     const long long paths = c.pixels() * c.spp;
     const int n = ds.n_leaves;
     const bool even = even_samples(c.spp);
+    if (ds.has_cones && paths > 1 << 22) return false;
     if (c.mode == PGPU_MODE_WHITTED) {
         if (!even) {
             const long long k = n <= 8 ? 512                // 1024 paths per bounce
@@ -1621,10 +1633,19 @@ static int32_t render_impl(pgpu_ctx* c, int32_t id, const pgpu_render_params* p,
     int launches = 1;
     double kms[KC_N] = {0};
     PGPU_CUDA(c, cudaEventRecord(c->ev0, c->stream));
-    cudaError_t e;
+    cudaError_t e = cudaSuccess;
     if (cfg.engine == PGPU_ENGINE_MEGAKERNEL || one_kernel_frame(*ds, cfg)) {
         *c->h_status = 0;
-        e = launch_megakernel(ds->view, cfg, d_out, d_m2, c->d_cnt, c->stream);
+        const float4* hits = nullptr;
+        if (cfg.engine == PGPU_ENGINE_WAVEFRONT && ds->has_cones) {
+            e = with_room(c, [&] {
+                return wavefront_camera_hits(*c->wf, ds->view, cfg, c->stream, &hits);
+            });
+            if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();   // one per lane then
+            else if (e != cudaSuccess) return cuda_fail(c, e, "camera packets launch");
+            if (hits) launches = 2;
+        }
+        e = launch_megakernel(ds->view, cfg, hits, d_out, d_m2, c->d_cnt, c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "megakernel launch");
     } else {
         *c->h_status = 0;
@@ -1715,7 +1736,8 @@ int32_t pgpu_render_tile(pgpu_ctx* c, int32_t id, const pgpu_render_params* p, i
     cfg.win[2] = tile_w;
     cfg.win[3] = tile_h;
     cfg.worker = true;
-    cudaError_t e = launch_megakernel(ds->view, cfg, d_out, nullptr, c->d_cnt, c->stream);
+    cudaError_t e = launch_megakernel(ds->view, cfg, nullptr, d_out, nullptr, c->d_cnt,
+                                      c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "megakernel launch");
     if (!dev_out)
         PGPU_CUDA(c, cudaMemcpyAsync(out_rgb, d_out, n3 * 4, cudaMemcpyDeviceToHost, c->stream));

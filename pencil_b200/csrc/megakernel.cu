@@ -13,13 +13,6 @@
 
 namespace pgpu {
 
-// Held to 64 registers (eight blocks of 128 threads per SM): more resident
-// warps hide more of the divergent paths' load latency than the spilled
-// words cost. Sphere-cloud frame 85.8 ms at the compiler's choice (96-128
-// registers) -> 73.4 at 72 -> 71.8 at 64; mesh frame 443.5 -> 378.0 ->
-// 382.3 ms.
-constexpr int kMkMinBlocks = 8;
-
 // megakernel_small.cu: launches that do not fill the GPU (*done), with a team of
 // lanes per pixel in the reference-exact mode.
 cudaError_t launch_mk_small(const SceneView& S, const PathParams& P, int G, long long threads,
@@ -45,8 +38,14 @@ static cudaError_t launch_mk(const SceneView& S, const PathParams& P, int G, lon
     return cudaGetLastError();
 }
 
-cudaError_t launch_megakernel(const SceneView& S, const RenderCfg& c, float* out, float* m2,
-                              unsigned long long* counters, cudaStream_t st) {
+// megakernel_found.cu
+cudaError_t launch_mk_found(const SceneView& S, const PathParams& P, int G, const float4* found,
+                            long long threads, float* out, float* m2, cudaStream_t st);
+
+// found: the closest hits of the camera rays, path by path (or null).
+cudaError_t launch_megakernel(const SceneView& S, const RenderCfg& c, const float4* found,
+                              float* out, float* m2, unsigned long long* counters,
+                              cudaStream_t st) {
     PathParams P{c.W, c.H, c.n, c.spp, c.depth, c.mode, c.rng, c.glass, c.soft, c.bias, c.salt,
                  c.sample_offset, c.mis ? 1 : 0, c.win[0], c.win[1], c.win[2], c.win[3],
                  c.worker ? 1 : 0};
@@ -57,6 +56,7 @@ cudaError_t launch_megakernel(const SceneView& S, const RenderCfg& c, float* out
         int lim = c.spp < 32 ? c.spp : 32;
         while (G * 2 <= lim) G *= 2;
     }
+    if (found) return launch_mk_found(S, P, G, found, c.pixels() * G, out, m2, st);
     const bool wide = !c.binary_tree;
 #define PGPU_MK_CASE(CNT, TR, SQ)                                                \
     if (c.count == CNT && tree == TR && seq == SQ)                               \

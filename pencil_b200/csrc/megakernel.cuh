@@ -1,7 +1,8 @@
 // megakernel.cuh - the path-per-thread kernel, shared by megakernel.cu (launches
-// that fill the GPU) and megakernel_small.cu (those that do not). Each has its
-// own instantiations: with both register budgets in one translation unit the
-// compiler no longer inlines the path loop into the larger launches' kernel
+// that fill the GPU), megakernel_small.cu (those that do not) and the two
+// megakernel_found files (the same for frames whose camera hits are given). Each
+// has its own instantiations: with both register budgets in one translation unit
+// the compiler no longer inlines the path loop into the larger launches' kernel
 // (100,000-sphere cloud, 3.7M paths: 21.2 -> 31.3 ms).
 #pragma once
 
@@ -16,10 +17,29 @@ constexpr int kMkBlock = 128;
 constexpr int kMkShared = 16;   // stack entries per thread kept in shared memory
 constexpr size_t kMkSmem = (size_t)kMkShared * kMkBlock * 8;
 
-template <bool COUNT, bool TREE, bool PIXEL_SEQ, bool WIDE, bool COOP, int MINB>
+// A launch that does not fill the GPU twice at four blocks per SM waits for its
+// longest paths rather than for issue slots, and gets the registers instead
+// (128, next to no spills). 8 / 4 blocks: 19,200 paths of three spheres 0.068 /
+// 0.062 ms, 12,288 among 20,000 spheres 0.334 / 0.271, 20,000 on a mesh 0.591 /
+// 0.512, 120,000 in a room 1.16 / 1.10; 230,400 among 20,000 spheres 0.69 / 0.79,
+// 262,144 on a mesh 1.70 / 1.93. The reference-exact tiles, which are always
+// that small, 1.81 / 1.47 and 0.42 / 0.31.
+constexpr int kMkSmallBlocks = 4;
+constexpr long long kMkSmallThreads = 2LL * 148 * kMkSmallBlocks * 128;
+
+// Held to 64 registers (eight blocks of 128 threads per SM) otherwise: more
+// resident warps hide more of the divergent paths' load latency than the spilled
+// words cost. Sphere-cloud frame 85.8 ms at the compiler's choice (96-128
+// registers) -> 73.4 at 72 -> 71.8 at 64; mesh frame 443.5 -> 378.0 ->
+// 382.3 ms.
+constexpr int kMkMinBlocks = 8;
+
+// FOUND: entry k of `found` is the closest hit of path k's camera ray.
+template <bool COUNT, bool TREE, bool PIXEL_SEQ, bool WIDE, bool COOP, int MINB, bool FOUND = false>
 __global__ void __launch_bounds__(kMkBlock, MINB)
 mk_render(SceneView S, PathParams P, int G, int per_warp, float* __restrict__ out,
-          float* __restrict__ m2, unsigned long long* __restrict__ counters) {
+          float* __restrict__ m2, unsigned long long* __restrict__ counters,
+          const float4* __restrict__ found = nullptr) {
     extern __shared__ int smem[];
     TravStack<kMkShared> stk;
     stk.sref = smem + threadIdx.x;
@@ -57,7 +77,12 @@ mk_render(SceneView S, PathParams P, int G, int per_warp, float* __restrict__ ou
                 Rng rng{path_seed(i, j, s + P.sample_offset, P.salt)};
                 float u, v;
                 sample_uv(i, j, s % P.n, s / P.n, P.W, P.H, P.n, rng, u, v, P.worker != 0);
-                V3 c = tr.template sample<TREE>(camera_ray(S.cam, u, v), rng);
+                V3 c;
+                if constexpr (FOUND)
+                    c = tr.template sample<TREE, true>(camera_ray(S.cam, u, v), rng,
+                                                       found + pix * P.spp + s);
+                else
+                    c = tr.template sample<TREE>(camera_ray(S.cam, u, v), rng);
                 acc = acc + c;
                 acc2 = acc2 + c * c;
             }

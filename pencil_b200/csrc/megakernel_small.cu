@@ -4,16 +4,6 @@
 
 namespace pgpu {
 
-// A launch that does not fill the GPU twice at four blocks per SM waits for its
-// longest paths rather than for issue slots, and gets the registers instead
-// (128, next to no spills). 8 / 4 blocks: 19,200 paths of three spheres 0.068 /
-// 0.062 ms, 12,288 among 20,000 spheres 0.334 / 0.271, 20,000 on a mesh 0.591 /
-// 0.512, 120,000 in a room 1.16 / 1.10; 230,400 among 20,000 spheres 0.69 / 0.79,
-// 262,144 on a mesh 1.70 / 1.93. The reference-exact tiles, which are always
-// that small, 1.81 / 1.47 and 0.42 / 0.31.
-constexpr int kMkSmallBlocks = 4;
-constexpr long long kMkSmallThreads = 2LL * 148 * kMkSmallBlocks * 128;
-
 // Lanes of a pixel's team in the reference-exact mode (Pencil's per-pixel
 // stream, both glass branches). A launch too small to fill the GPU (a worker's
 // 64x64 tile has 4096 pixels) ends with its longest path, a serial chain of node

@@ -603,14 +603,16 @@ struct Tracer {
 
     // One camera sample. TREE: both glass branches (Pencil's recursion, used
     // with the per-pixel RNG for bit-level comparison); otherwise the
-    // Fresnel-split single-ray continuation.
-    template <bool TREE>
-    __device__ V3 sample(Ray r, Rng& rng) {
+    // Fresnel-split single-ray continuation (FOUND: `found` holds the camera
+    // ray's closest hit, a wavefront packet's).
+    template <bool TREE, bool FOUND = false>
+    __device__ V3 sample(Ray r, Rng& rng, const float4* found = nullptr) {
+        static_assert(!(TREE && FOUND), "both glass branches trace their own camera rays");
         if (P.mode == kModeWhitted) {
             if (TREE) return whitted_tree(r, P.depth, rng, false, nullptr, nullptr);
-            return split_path(r, rng, true);
+            return split_path<FOUND>(r, rng, true, found);
         }
-        if (!TREE) return split_path(r, rng, false);
+        if (!TREE) return split_path<FOUND>(r, rng, false, found);
         // trace_path with Pencil's glass recursion
         if (COUNT) rc.ref++;
         V3 T = v3(1, 1, 1), rad = v3(0, 0, 0);
@@ -720,7 +722,8 @@ struct Tracer {
 
     // Single-ray path (Fresnel-split glass): shade_vertex with every shadow
     // ray resolved on the spot.
-    __device__ V3 split_path(Ray r, Rng& rng, bool whitted) {
+    template <bool FOUND>
+    __device__ V3 split_path(Ray r, Rng& rng, bool whitted, const float4* camera) {
         PathState ps;
         ps.ray = r;
         ps.T = v3(1, 1, 1);
@@ -732,7 +735,16 @@ struct Tracer {
         bool alive = ps.depth > 0;
         while (alive) {
             Hit h;
-            bool found = closest(ps.ray, h) >= 0;
+            bool found;
+            if (FOUND && camera) {
+                const float4 f = __ldcs(camera);
+                camera = nullptr;
+                found = __float_as_int(f.z) >= 0;
+                if (found)
+                    make_hit(S, __float_as_int(f.y), __float_as_int(f.z), ps.ray, 1e-4f, f.x, h);
+            } else {
+                found = closest(ps.ray, h) >= 0;
+            }
             InlineNee emit{*this};
             alive = shade_vertex(S, P, ps, found, h, emit);
             emit.acc.finish(ps.L, emit.tail, emit.w, emit.s);

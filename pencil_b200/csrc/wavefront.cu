@@ -1651,6 +1651,33 @@ cudaError_t wavefront_adjoint(WfScratch& W, const SceneView& view,
     return e;
 }
 
+// The closest hits of a frame's camera rays, traced as the queues trace them:
+// entry k of *hits is path k's (t, ref, leaf slot; slot -1: none). Null where the
+// scene has no camera-relative nodes, whose frames trace them one per lane.
+cudaError_t wavefront_camera_hits(WfScratch& W, const SceneView& view, const RenderCfg& cfg,
+                                  cudaStream_t st, const float4** hits) {
+    *hits = nullptr;
+    if (!packets_for(view)) return cudaSuccess;
+    const int Q = (int)(cfg.pixels() * cfg.spp);
+    cudaError_t e = ensure_scratch(W, Q, 1, 1, 1, 1);
+    if (e != cudaSuccess) return e;
+    WfArgs A = W.args;
+    A.n_jobs = 1;
+    A.view0 = view;
+    A.job0.P = PathParams{cfg.W, cfg.H, cfg.n, cfg.spp, cfg.depth, cfg.mode, cfg.rng, cfg.glass,
+                          cfg.soft, cfg.bias, cfg.salt, cfg.sample_offset, cfg.mis ? 1 : 0,
+                          cfg.win[0], cfg.win[1], cfg.win[2], cfg.win[3], 0};
+    A.job0.view = 0;
+    A.job0.path_off = A.job0.pix_off = 0;
+    WfOccupancy occ;
+    if ((e = occupancy<false, true, true>(occ)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(A.counts, 0, 3 * kOctants * 4, st)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(A.work, 0, 3 * 3 * 4, st)) != cudaSuccess) return e;
+    wf_camera<false, true, true><<<occ.grid_packet, kWfBlock, 0, st>>>(A, 0, Q);
+    if ((e = cudaGetLastError()) == cudaSuccess) *hits = A.hit;
+    return e;
+}
+
 void wavefront_release(WfScratch& W) {
     if (W.graph) cudaGraphExecDestroy(W.graph);
     W.graph = nullptr;
