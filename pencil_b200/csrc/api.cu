@@ -1436,21 +1436,22 @@ int run_wavefront(pgpu_ctx* c, const std::vector<DeviceScene*>& scenes,
     return PGPU_OK;
 }
 
-// Whether a pixel's samples keep its lanes of one kernel busy alike: 1, 4, 16 or
-// 64 do, 9 (two turns of 8 lanes), 25, 36 or 49 keep a fifth to a half idle.
-static bool even_samples(int spp) {
+// The turns of its lanes in one kernel over a pixel's samples: 1 for 1, 4, 16 or
+// 64 samples, 1.3 for 25 or 49 (32 turns of 16 lanes, 64 of 32), 1.8 for 9 or 36.
+static double lane_turns(int spp) {
     int lanes = 1;
     while (lanes * 2 <= std::min(spp, 32)) lanes *= 2;
-    return (spp + lanes - 1) / lanes * lanes * 4 <= spp * 5;
+    return (double)((spp + lanes - 1) / lanes * lanes) / spp;
 }
+static bool even_samples(int spp) { return lane_turns(spp) <= 1.25; }
 
 // Whether a frame of the wavefront engine runs as one kernel, a thread per
 // path, instead of the queued kernels: the same image bit for bit. (The sides of
 // cones lie outside the box that the reference gives them, so that the walk's
 // order decides which rays find them, and packets take another than lanes of
 // their own. Frames of scenes with cones therefore have their camera rays
-// traced as the queues trace them, first, where one chunk of the queues would
-// hold them; in 4 of 110 rooms that showed, in 2 to 22 pixels, where the packets
+// traced as the queues trace them, first, where the packets are the queues':
+// every chunk is whole packets, or there is one chunk; in 4 of 110 rooms that showed, in 2 to 22 pixels, where the packets
 // agree with the reference's order.) Queues pay three kernels a bounce,
 // each as long as its longest ray; one kernel pays once, but its warps run
 // their paths' parts in turn, which costs more the more rays there are and the
@@ -1495,8 +1496,12 @@ static bool even_samples(int spp) {
 // and depth 10, 103: 0.90 at 263k, 1.32 at 1.0M, 253: 1.09, 1.53; matte: 312
 // spheres 0.71 at 66k, 1.08 at 263k, 338 triangles 0.98 at 1.0M, 5,138: 0.73 at
 // 66k, 1.10 at 263k, 82,000: 0.69, 1.20; 20,000 spheres of every kind 0.72, 1.36.
-// Path tracing: walls 1.22-1.42 at 66k and depth 4 (even 0.88-0.96), 0.93-1.09 at
-// 16k; three spheres 1.16 at 263k (even 0.84); open scenes as above.
+// 25 samples: rooms of 23 and 63 0.79 and 0.84 at 1.1M and depth 4, 0.91 and 0.96 at
+// 4.2M, 103: 1.06, 1.18, at depth 10 0.78, 1.07; matte: 312 spheres 0.93, 0.97,
+// 82,000 triangles 0.76 at 65k, 1.36 at 1.1M.
+// Path tracing: walls 1.11-1.31 at 66k and depth 4 (even 0.88-0.96), 0.99-1.09 at
+// 16k; with cubes, cylinders and cones 1.42-2.0 at 66k, 0.93-1.15 at 16k, 0.59-0.65 at 16k
+// and depth 10; three spheres 1.16 at 263k (even 0.84); open scenes as above.
 // Frames that count, profile or set a launch parameter keep the queues.
 static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
     if (c.count || c.profile || !c.packets || c.queue_capacity || c.sort_key || c.refill ||
@@ -1505,13 +1510,14 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
     const long long paths = c.pixels() * c.spp;
     const int n = ds.n_leaves;
     const bool even = even_samples(c.spp);
-    if (ds.has_cones && paths > 1 << 22) return false;
+    if (ds.has_cones && paths > ((c.spp & (c.spp - 1)) == 0 ? 1 << 24 : 1 << 22)) return false;
     if (c.mode == PGPU_MODE_WHITTED) {
         if (!even) {
             const long long k = n <= 8 ? 512                // 1024 paths per bounce
                 : n <= (ds.mostly_triangles ? 512 : ds.has_reflective ? 64 : 8) ? 256
                 : n <= 128 && ds.has_reflective ? 100 : n <= 8192 ? 64 : 32;
-            if (paths > k * 1024 * std::min(c.depth, 16)) return false;
+            const int mild = lane_turns(c.spp) <= 4.0 / 3.0 ? 3 : 1;
+            if (paths > k * mild * 1024 * std::min(c.depth, 16)) return false;
         }
         if (!ds.has_reflective) return n <= 1024 || ds.mostly_triangles || paths <= 1 << 18;
         if (n > 256) return paths <= (n <= 65536 || ds.mostly_triangles ? 1 << 18 : 1 << 17);
@@ -1521,7 +1527,10 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
             if (l.kind != PGPU_LIGHT_QUAD) records += l.radius > 0.0f ? c.soft : 1;
         if (n <= 128 && c.spp >= (n <= 64 ? 4 : 16)) return true;
         const long long each = n <= 64 ? 1 << 18 : n <= 128 ? 1 << 17 : 3 << 15;
-        return paths <= each * std::max(records, 1LL) * (c.spp >= 16 ? 8 : c.spp >= 4 ? 2 : 1);
+        // (measured at depth 4; at 10, 103 primitives 0.72 at 1.0M, 0.99 at 4.2M, 253: 0.94, 1.33)
+        return paths * 4 <= each * std::max(records, 1LL) *
+                                (c.spp >= 16 ? 8 : c.spp >= 4 ? 2 : 1) *
+                                std::min(std::max(c.depth, 4), 16);
     }
     long long rays = 1;                     // of a path-traced vertex
     for (const DevLight& l : ds.lights) rays += l.is_emissive ? 0 : 1;
@@ -1536,7 +1545,7 @@ static bool one_kernel_frame(const DeviceScene& ds, const RenderCfg& c) {
         per = n <= 1024 || ds.mostly_triangles ? 128 : n <= 8192 ? 32 : n <= 32768 ? 16 : 12;
         rays = 1;
     }
-    if (!even && n > 8 && (ds.has_long_kinds || ds.has_walls)) rays *= 4;
+    if (!even && n > 8) rays *= ds.has_long_kinds ? 2 : ds.has_walls ? 3 : 1;
     return paths * rays <= per * 1024 * std::min(std::max(c.depth, 4), 16);
 }
 

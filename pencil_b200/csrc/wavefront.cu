@@ -1671,8 +1671,9 @@ cudaError_t wavefront_camera_hits(WfScratch& W, const SceneView& view, const Ren
     A.job0.path_off = A.job0.pix_off = 0;
     WfOccupancy occ;
     if ((e = occupancy<false, true, true>(occ)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(A.counts, 0, 3 * kOctants * 4, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(A.work, 0, 3 * 3 * 4, st)) != cudaSuccess) return e;
+    // the queue's count and the cursor, which carve() lays one after the other
+    const size_t clear = reinterpret_cast<char*>(A.work + 1) - reinterpret_cast<char*>(A.counts);
+    if ((e = cudaMemsetAsync(A.counts, 0, clear, st)) != cudaSuccess) return e;
     wf_camera<false, true, true><<<occ.grid_packet, kWfBlock, 0, st>>>(A, 0, Q);
     if ((e = cudaGetLastError()) == cudaSuccess) *hits = A.hit;
     return e;

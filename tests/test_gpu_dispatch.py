@@ -134,11 +134,11 @@ def test_frames_of_one_kernel_at_any_size(gpu, name):
 # samples that a pixel's lanes share unevenly (9 of 8 lanes, 25 of 16)
 @pytest.mark.parametrize("name,pathtrace,depth,samples,size", [
     ("spheres", True, 4, 3, (182, 120)), ("spheres", False, 3, 3, (512, 341)),
-    ("box338", True, 4, 3, (64, 24)), ("box338", False, 3, 3, (256, 341)),
-    ("room123", False, 2, 3, (256, 88)), ("room20", False, 2, 5, (256, 81)),
+    ("box338", True, 4, 3, (64, 33)), ("room20", True, 4, 3, (64, 35)),
+    ("box338", False, 3, 3, (256, 341)), ("room123", False, 2, 3, (256, 88)), ("room20", False, 2, 5, (256, 245)),
     ("matte20000", False, 4, 3, (128, 113)), ("lone5120", False, 4, 3, (128, 227)),
-    ("cloud300", True, 4, 3, (256, 227))])
-def test_lines_of_uneven_samples(gpu, name, pathtrace, depth, samples, size):
+    ("cloud300", True, 4, 3, (256, 227)), ("room123", False, 8, 1, (1024, 1536))])
+def test_lines_of_uneven_samples_and_depth(gpu, name, pathtrace, depth, samples, size):
     test_both_sides_of_each_line(gpu, name, pathtrace, depth, samples, size)
 
 
